@@ -64,7 +64,7 @@ struct GemmArgs {
   // and on whole tiles afterwards, so a partial is ready long before its finisher asks for it.
   int sk_tiles;
   float* sk_scratch;    // per pair 2 x 128 x 256 floats (256 KiB)
-  uint32_t* sk_flags;   // per pair 8 words (one per epilogue warp of the pair), holding the last epoch written
+  uint32_t* sk_flags;   // per pair 16 words (one per epilogue warp of the pair), holding the last epoch written
   uint32_t sk_epoch;    // differs from launch to launch on the same scratch
   // ---- tiles handed out at run time (CTA-pair form; sched_counter == nullptr: static round-robin)
   // A persistent kernel that deals its tiles out in advance assumes that all its CTA pairs start
@@ -87,7 +87,7 @@ struct GemmArgs {
 
 // Bytes of sk_scratch / words of sk_flags needed for `pairs` CTA pairs.
 constexpr size_t kGemmSkScratchBytesPerPair = 2 * 128 * 256 * sizeof(float);
-constexpr size_t kGemmSkFlagsPerPair = 8;
+constexpr size_t kGemmSkFlagsPerPair = 16;
 
 // How many leading tiles launch_gemm_sm100 would split along K for this shape on `sm_count` SMs
 // (0: none).  The caller provides scratch for sm_count / 2 pairs when this is non-zero.

@@ -503,18 +503,28 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // holding 64 consecutive rows of the operand; blocks 8 KiB apart).  The MMA reads either
 // through its shared-memory descriptor, so no transposing copy exists anywhere.
 //
-// Epilogue.  Every epilogue warp owns 32 accumulator rows.  It reads 64 columns from TMEM,
-// adds the bias, rounds to bf16, writes the 32x64 slab into its own 4 KiB piece of shared
-// memory in the 128-byte-swizzled layout and hands it to the copy engine as one tiled TMA
-// store (which also clips rows and columns beyond M and N); two pieces per warp alternate.
+// Epilogue.  Eight warps: warp w owns 32 accumulator rows (a warp may only read the quarter
+// w % 4 of the TMEM lanes) and one half of the 256 columns.  It reads 64 columns from TMEM, adds
+// the bias, rounds to bf16, writes the 32x64 slab into its own 4 KiB piece of shared memory in the
+// 128-byte-swizzled layout and hands it to the copy engine as one tiled TMA store (which also
+// clips rows and columns beyond M and N).  The work is a chain of latencies (TMEM, shared memory,
+// proxy fence), so two warps per scheduler, each with half the slabs, halve it, and the options
+// (activation, gelu' factor) are decided once per slab instead of inside the loops.  The bias of a
+// slab is fetched before the accumulator is ready, one bf16 pair per lane, and read back as a
+// broadcast from shared memory.  Measured against four warps with two pieces each (kernel time): 4096 x 4096 x
+// 1024 with bias 50.5 -> 33.9 us, with bias and GELU 65.5 -> 40.7 us (there the epilogue of a tile took longer
+// than its main loop), 256 x 768 x 256 13.0 -> 7.5 us together with the work done between the halves of the
+// first cluster barrier and the relaxed last one.
 constexpr int kStages2 = 6;
 constexpr uint32_t kHalfBytes = 128 * BK * 2;              // 16 KiB: 128 rows x 64 bf16
 constexpr uint32_t kStage2Bytes = 2 * kHalfBytes;          // A half + W half
+constexpr int kEpiWarps = 8;                               // per CTA: two per quarter of the accumulator's rows
+constexpr int kGemm2Threads = 64 + 32 * kEpiWarps;
 constexpr uint32_t kEpiOff = kStages2 * kStage2Bytes;      // 196,608
-constexpr uint32_t kEpiSlabBytes = 32 * 64 * 2;            // 4 KiB: 32 rows x 64 bf16
-constexpr uint32_t kEpiWarpBytes = 2 * kEpiSlabBytes;      // two slabs per epilogue warp
-constexpr uint32_t kBar2Off = kEpiOff + 4 * kEpiWarpBytes; // 229,376
-constexpr uint32_t kGemm2Smem = kBar2Off + 256 + 1024;     // 230,656 of the 232,448 a CTA may have
+constexpr uint32_t kEpiSlabBytes = 32 * 64 * 2;            // 4 KiB: 32 rows x 64 bf16, one slab per epilogue warp
+constexpr uint32_t kEpiBiasBytes = 64 * 2;                 // the bias of one slab's columns, per epilogue warp
+constexpr uint32_t kBar2Off = kEpiOff + kEpiWarps * (kEpiSlabBytes + kEpiBiasBytes);   // 230,400
+constexpr uint32_t kGemm2Smem = kBar2Off + 256 + 1024;     // 231,680 of the 232,448 a CTA may have
 static_assert(kBulkSmemBytes <= kBar2Off + 256, "the gatherer's copy ring must fit");
 constexpr uint32_t kIdesc2 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 
@@ -536,15 +546,19 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// The cluster barrier in two halves, so that independent work fits between them.  It is also a barrier of
+// the CTA.  The relaxed arrival orders execution only: what other threads wrote is not made visible by it.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Address of the same shared-memory variable in another CTA of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
+}
+__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
   asm volatile(
@@ -576,37 +590,24 @@ __device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t da, uint
 __device__ __forceinline__ void mma_commit_pair(uint32_t bar_cluster_addr) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
+// Arrival on a barrier of either CTA that publishes no memory (an accumulator that has been read into registers is
+// handed back: tcgen05.wait::ld and the fence before this order that).  A release at cluster scope in its place
+// waits for the thread's copy-engine store too: about 2000 cycles per tile.
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t bar_cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-// Round eight accumulator values (+ bias) to bf16; returns them packed, and gelu() of the
-// rounded values in `g` when ACT.
-template <bool ACT>
-__device__ __forceinline__ uint4 pack8(const uint32_t* r, const float* b, uint4* g) {
-  uint32_t w[4], gg[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float x0 = __uint_as_float(r[2 * e]) + b[2 * e], x1 = __uint_as_float(r[2 * e + 1]) + b[2 * e + 1];
-    __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-    w[e] = *reinterpret_cast<uint32_t*>(&h);
-    if (ACT) {
-      __nv_bfloat162 hg = __floats2bfloat162_rn(gelu_tanh(__low2float(h)), gelu_tanh(__high2float(h)));
-      gg[e] = *reinterpret_cast<uint32_t*>(&hg);
-    }
-  }
-  if (ACT) *g = make_uint4(gg[0], gg[1], gg[2], gg[3]);
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
 // ---- tiles drawn at run time.  The producer thread of the leader CTA draws the next tile number
 // from the global counter and hands it to every other role of the pair (the peer CTA's producer,
-// the MMA issuer, the eight epilogue warps) through a four-slot ring in each CTA's shared memory:
+// the MMA issuer, the epilogue warps) through a four-slot ring in each CTA's shared memory:
 // value written into both CTAs, then one arrival on each CTA's `ready` barrier of the slot; a
 // reader copies the value and arrives on the leader's `taken` barrier at once, so a slot is free
-// again as soon as all ten readers have looked at it.
+// again as soon as all readers have looked at it.
 constexpr int kSchedSlots = 4;
-constexpr uint32_t kSchedReaders = 10;     // peer producer, MMA issuer, 2 x 4 epilogue warps
+constexpr uint32_t kSchedReaders = 2 + 2 * kEpiWarps;     // peer producer, MMA issuer, the epilogue warps of both CTAs
 constexpr int kSchedDone = -1;
 
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
@@ -664,20 +665,22 @@ __device__ __forceinline__ bool sched_read(const SchedRing& r, uint32_t n, volat
 // run of the k-block sequence of the leading sk_tiles tiles (see GemmArgs), then whole tiles
 // sk_tiles + pair, + npairs, ...  Producer, MMA issuer and epilogue walk the same sequence.
 struct WorkIter {
-  long long cur, end;     // position in the k-block sequence of the split tiles
+  int cur, end;           // position in the k-block sequence of the split tiles (the host keeps it within 31 bits)
   int nkb, next_tile, total, stride;
   __device__ __forceinline__ WorkIter(int pair, int npairs, int total_, int nkb_, int sk_tiles)
-      : nkb(nkb_), next_tile(sk_tiles + pair), total(total_), stride(npairs) {
-    const long long I = (long long)sk_tiles * nkb_;
-    cur = I * pair / npairs;
-    end = I * (pair + 1) / npairs;
+      : cur(0), end(0), nkb(nkb_), next_tile(sk_tiles + pair), total(total_), stride(npairs) {
+    if (sk_tiles > 0) {
+      const int I = sk_tiles * nkb_;
+      cur = (int)((unsigned)(I * pair) / (unsigned)npairs);
+      end = (int)((unsigned)(I * (pair + 1)) / (unsigned)npairs);
+    }
   }
   __device__ __forceinline__ bool next(int* tile, int* kb0, int* kb1) {
     if (cur < end) {
-      const int t = (int)(cur / nkb);
-      const int k0 = (int)(cur - (long long)t * nkb);
-      const long long left = end - cur;
-      const int k1 = (long long)(nkb - k0) <= left ? nkb : (int)(k0 + left);
+      const int t = cur / nkb;
+      const int k0 = cur - t * nkb;
+      const int left = end - cur;
+      const int k1 = nkb - k0 <= left ? nkb : k0 + left;
       *tile = t;
       *kb0 = k0;
       *kb1 = k1;
@@ -695,7 +698,60 @@ struct WorkIter {
   }
 };
 // The pair whose run of the split sequence (I k-blocks over G pairs) holds k-block i.
-__device__ __forceinline__ int sk_pair_of(long long i, long long I, int G) { return (int)(((i + 1) * G + I - 1) / I) - 1; }
+__device__ __forceinline__ int sk_pair_of(int i, int I, int G) { return (int)((unsigned)((i + 1) * G + I - 1) / (unsigned)I) - 1; }
+
+// One 32x64 slab of the epilogue: lane `lane` holds the 64 fp32 results of its row in r.  Rounds them
+// to bf16 and writes them to the warp's piece of shared memory in the 128-byte-swizzled layout (16-byte
+// chunk c of row l at chunk c ^ (l % 8)).  bias_s: this slab's 64 bias values in shared memory, or nullptr.
+// KEEP: the packed pairs stay in r[0..32) for a second output.
+// Both halves of a pair of fp32 values in one instruction.
+__device__ __forceinline__ void add_pair(uint32_t& x, uint32_t& y, uint32_t bx, uint32_t by) {
+  asm("{\n\t.reg .b64 p, q;\n\t"
+      "mov.b64 p, {%0, %1};\n\t"
+      "mov.b64 q, {%2, %3};\n\t"
+      "add.rn.f32x2 p, p, q;\n\t"
+      "mov.b64 {%0, %1}, p;\n\t}"
+      : "+r"(x), "+r"(y)
+      : "r"(bx), "r"(by));
+}
+template <bool BIAS, bool KEEP>
+__device__ __forceinline__ void slab_to_smem(uint32_t (&r)[64], unsigned char* buf, const unsigned char* bias_s, int lane) {
+  const uint32_t sw = (uint32_t)(lane & 7);
+  unsigned char* row = buf + lane * 128;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    if (BIAS) {
+      const uint4 q = *reinterpret_cast<const uint4*>(bias_s + c * 16);
+      const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) add_pair(r[c * 8 + 2 * e], r[c * 8 + 2 * e + 1], qw[e] << 16, qw[e] & 0xffff0000u);
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[c * 8 + 2 * e]), __uint_as_float(r[c * 8 + 2 * e + 1]));
+      w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      if (KEEP) r[c * 4 + e] = w[e];             // a pair is read before its place is written
+    }
+    *reinterpret_cast<uint4*>(row + (((uint32_t)c ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+// gelu() of the 32 packed bf16 pairs that slab_to_smem left in r[0..32), into the same layout.
+__device__ __forceinline__ void slab_gelu_to_smem(const uint32_t (&r)[64], unsigned char* buf, int lane) {
+  const uint32_t sw = (uint32_t)(lane & 7);
+  unsigned char* row = buf + lane * 128;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t v = r[c * 4 + e];
+      const __nv_bfloat162 h = __floats2bfloat162_rn(gelu_tanh(__uint_as_float(v << 16)), gelu_tanh(__uint_as_float(v & 0xffff0000u)));
+      w[e] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(row + (((uint32_t)c ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
 
 // WIDE: the unit of work is two vertically adjacent 256 x 256 tiles that share their W half:
 // a stage holds two A halves and one W half (48 KiB, four stages), the MMA issuer feeds both
@@ -703,7 +759,7 @@ __device__ __forceinline__ int sk_pair_of(long long i, long long I, int G) { ret
 // fewer operand bytes come from L2 per FLOP; the price is that both accumulators belong to one
 // unit, so the epilogue of a unit overlaps only the first k-blocks of the next.
 template <bool A_MN, bool B_MN, bool WIDE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
     gemm_sm100_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                            const __grid_constant__ CUtensorMap tmWown, const __grid_constant__ CUtensorMap tmC,
                            const __grid_constant__ CUtensorMap tmAct, const __grid_constant__ GemmArgs a) {
@@ -730,6 +786,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   ring.tile = reinterpret_cast<int*>(ring.taken + kSchedSlots);
   const bool dynamic = a.sched_counter != nullptr;
 
+  if (threadIdx.x == 64) {
+    // the descriptors are on their way while the barriers are set up
+    prefetch_tensormap(&tmA);
+    prefetch_tensormap(&tmW);
+    prefetch_tensormap(&tmC);
+    if (a.panel_flags != nullptr) prefetch_tensormap(&tmWown);
+    if (a.act_out != nullptr) prefetch_tensormap(&tmAct);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages2; ++s) {
       mbar_init(full + s, 1);
@@ -737,7 +801,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(tmem_full + i, 1);
-      mbar_init(tmem_empty + i, 8);        // four epilogue warps of each CTA
+      mbar_init(tmem_empty + i, 2 * kEpiWarps);        // the epilogue warps of both CTAs
     }
     for (int i = 0; i < kSchedSlots; ++i) {
       mbar_init(ring.ready + i, 1);
@@ -752,11 +816,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();                       // both CTAs' barriers exist before anyone signals across
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  __syncwarp();
+  cluster_arrive();
 
+  // Between the halves of the barrier: this thread's first piece of work.  Its divisions and the first touch of
+  // the launch parameters take longer than the barrier.
   constexpr int NST = WIDE ? 4 : kStages2;                                  // stages in flight
   constexpr uint32_t SB = WIDE ? 3 * kHalfBytes : kStage2Bytes;             // bytes of one stage in one CTA
   constexpr uint32_t W_OFF = WIDE ? 2 * kHalfBytes : kHalfBytes;            // where the W half sits in a stage
@@ -794,15 +858,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     *n_idx = fused ? ((me + q / tpr) % P) * tpr + q % tpr : q;
   };
 
+  WorkIter work(pair, npairs, total, nkb, a.sk_tiles);
+  int t = 0, kb0 = 0, kb1 = nkb, m_first = 0, n_first = 0;
+  bool first = !dynamic && work.next(&t, &kb0, &kb1);      // the first item is already in t, kb0, kb1
+  const bool any = dynamic || first;
+  if (first) decode(t, &m_first, &n_first);
+  asm volatile("" : "+r"(t), "+r"(kb0), "+r"(kb1), "+r"(m_first), "+r"(n_first));     // computed here, not after the wait
+  auto next_static = [&]() -> bool {
+    if (first) {
+      first = false;
+      return true;
+    }
+    return any && work.next(&t, &kb0, &kb1);
+  };
+
+  cluster_wait();                           // both CTAs' barriers exist before anyone signals across
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
   if (warp == 0 && lane == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     uint32_t it = 0;
     bool ok = true;
-    WorkIter work(pair, npairs, total, nkb, a.sk_tiles);
-    int t, kb0, kb1;
     uint32_t drawn = 0;
     auto next_item = [&]() -> bool {
-      if (!dynamic) return work.next(&t, &kb0, &kb1);
+      if (!dynamic) return next_static();
       kb0 = 0;
       kb1 = nkb;
       const bool got = leader ? sched_draw(a, ring, drawn, total, abort_flag, &t) : sched_read(ring, drawn, abort_flag, &t);
@@ -814,9 +894,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       }
       return t != kSchedDone;
     };
+    bool decoded = !dynamic;
     while (ok && next_item()) {
-      int m_idx, n_idx;
-      decode(t, &m_idx, &n_idx);
+      int m_idx = m_first, n_idx = n_first;
+      if (!decoded) decode(t, &m_idx, &n_idx);
+      decoded = false;
       const CUtensorMap* wmap = &tmW;
       int wy = n_idx * 256 + (int)rank * 128;
       if (fused) {
@@ -869,7 +951,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
         else tma_load_2d_pair(sa + W_OFF, wmap, kb * BK, wy, bar);
       }
     }
-    if (!ok) *abort_flag = 1;
+    // Tail: see every signal that the other CTA still sends to this one (stages given back, ring slots taken),
+    // so that the CTAs may leave after a barrier that orders execution only.
+    for (uint32_t n = it > (uint32_t)NST ? it - NST : 0; ok && n < it; ++n)
+      ok = gemm_wait(empty + n % NST, (n / NST) & 1u, abort_flag);
+    if (leader)
+      for (uint32_t n = drawn > (uint32_t)kSchedSlots ? drawn - kSchedSlots : 0; ok && n < drawn; ++n)
+        ok = sched_wait(ring.taken + n % kSchedSlots, (n / kSchedSlots) & 1u, abort_flag);
+    if (!ok) {
+      atomicCAS(a.error, 0, kErrProducer);
+      *abort_flag = 1;
+    }
   } else if (warp == 1 && lane == 0 && leader) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     constexpr uint32_t idesc = kIdesc2 | (A_MN ? (1u << 15) : 0u) | (B_MN ? (1u << 16) : 0u);
@@ -877,10 +969,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     constexpr uint64_t b_step = B_MN ? (2048 >> 4) : (32 >> 4);
     uint32_t it = 0, tile_count = 0, draws = 0;
     bool ok = true;
-    WorkIter work(pair, npairs, total, nkb, a.sk_tiles);
-    int t, kb0, kb1;
     auto next_item = [&]() -> bool {
-      if (!dynamic) return work.next(&t, &kb0, &kb1);
+      if (!dynamic) return next_static();
       kb0 = 0;
       kb1 = nkb;
       if (!sched_read(ring, draws++, abort_flag, &t)) {      // draws, not tiles: a unit of two tiles is one draw
@@ -932,6 +1022,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
         mma_commit_pair(map_to_cta(fb1, 1));
       }
     }
+    // Tail: every accumulator has been handed back (arrivals from the other CTA among them).
+    for (uint32_t n = tile_count > 2 ? tile_count - 2 : 0; ok && n < tile_count; ++n)
+      ok = gemm_wait(tmem_empty + (n & 1u), (n >> 1) & 1u, abort_flag);
     if (!ok) {
       atomicCAS(a.error, 0, kErrMma);
       *abort_flag = 1;
@@ -941,21 +1034,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     uint32_t tile_count = 0;
     bool ok = true;
     const int q = warp & 3;                     // the quarter of the TMEM lanes this warp may read
+    const int half = (warp - 2) >> 2;           // columns [128 * half, +128) of a tile
     const int lane_base = q * 32;
-    unsigned char* ebuf = smem + kEpiOff + (size_t)q * kEpiWarpBytes;
+    unsigned char* buf = smem + kEpiOff + (size_t)(warp - 2) * kEpiSlabBytes;
+    unsigned char* bias_s = smem + kEpiOff + (size_t)kEpiWarps * kEpiSlabBytes + (size_t)(warp - 2) * kEpiBiasBytes;
     const bool has_act = a.act_out != nullptr;
     const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(a.bias);
-    const uint32_t sw = (uint32_t)(lane & 7);   // 128-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r % 8)
-    uint32_t nstore = 0;                        // slabs stored so far: picks the piece, across tiles too
     uint32_t draws = 0;                         // tiles (or units) taken from the run-time scheduler so far
-    WorkIter work(pair, npairs, total, nkb, a.sk_tiles);
-    const long long sk_I = (long long)a.sk_tiles * nkb;
-    // this warp's 32 x 256 fp32 block inside a pair's scratch slot, and its flag word
-    const size_t sk_warp = ((size_t)rank * 4 + (size_t)q) * (32 * 256);
-    const uint32_t sk_word = rank * 4 + (uint32_t)q;
-    int t, kb0, kb1;
+    const int sk_I = a.sk_tiles * nkb;
+    // this warp's 32 x 128 fp32 block inside a pair's scratch slot, and its flag word
+    const uint32_t sk_word = (rank * 4 + (uint32_t)q) * 2 + (uint32_t)half;
+    const size_t sk_warp = (size_t)sk_word * (32 * 128);
     auto next_item = [&]() -> bool {
-      if (!dynamic) return work.next(&t, &kb0, &kb1);
+      if (!dynamic) return next_static();
       kb0 = 0;
       kb1 = nkb;
       int got = 1;
@@ -985,6 +1076,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       decode(t, &m_idx, &n_idx);
       if (WIDE) m_idx = 2 * m_idx + sub;
       const uint32_t acc = tile_count & 1u, acc_ph = (tile_count >> 1) & 1u;
+      const int colw = n_idx * 256 + half * 128;                       // first of this warp's 128 columns
+      // the bias of both slabs, two columns per lane, on its way while the accumulator is being formed
+      uint32_t bias_q[2] = {0u, 0u};
+      if (bias != nullptr) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s)                                    // N % 8 == 0: a pair is inside or outside as a whole
+          if (colw + s * 64 + 2 * lane < a.N) bias_q[s] = __ldg(reinterpret_cast<const uint32_t*>(bias + colw + s * 64) + lane);
+      }
       // one lane polls the barrier (with a pause between polls: an accumulator takes microseconds),
       // the others wait at the shuffle: 124 fewer threads hammering shared memory beside the MMAs
       if (lane == 0) ok = gemm_wait_relaxed(tmem_full + acc, acc_ph, abort_flag);
@@ -992,12 +1091,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       if (!ok) break;
       tc_fence_after();
       const int row0 = m_idx * 256 + (int)rank * 128 + lane_base;     // first of this warp's 32 rows
-      const uint32_t t_base = tmem_base + acc * BN + ((uint32_t)lane_base << 16);
+      const uint32_t t_base = tmem_base + acc * BN + (uint32_t)(half * 128) + ((uint32_t)lane_base << 16);
       const bool partial_only = kb0 > 0;                               // a piece of a tile somebody else finishes
       int first_helper = 0, last_helper = -1;                          // pairs whose partial sums this tile still needs
       if (kb0 == 0 && kb1 < nkb) {
         first_helper = pair + 1;
-        last_helper = sk_pair_of((long long)(t + 1) * nkb - 1, sk_I, npairs);
+        last_helper = sk_pair_of((t + 1) * nkb - 1, sk_I, npairs);
         for (int h = first_helper; h <= last_helper && ok; ++h) {
           if (lane == 0) {
             const uint32_t* flag = a.sk_flags + (size_t)h * kGemmSkFlagsPerPair + sk_word;
@@ -1019,21 +1118,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
           // hand the accumulator back so that the other roles can drain, then give up
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty + acc), 0));
+          if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(tmem_empty + acc), 0));
           break;
         }
       }
 #pragma unroll 1
-      for (int slab = 0; slab < BN / 64; ++slab) {
+      for (int slab = 0; slab < 2; ++slab) {
         uint32_t r[64];
         tmem_ld32(t_base + slab * 64, r);
         tmem_ld32(t_base + slab * 64 + 32, r + 32);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (slab == BN / 64 - 1) {
+        if (slab == 1) {
           // the accumulator is in registers: hand it back to the MMA issuer before storing
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty + acc), 0));
+          if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(tmem_empty + acc), 0));
         }
         if (partial_only) {
           // fp32 partial sums to this pair's scratch slot: float4 j of lane l at (j * 32 + l), so a warp's store is contiguous
@@ -1042,7 +1141,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
           for (int j = 0; j < 16; ++j)
             __stcg(dst + j * 32, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
                                              __uint_as_float(r[4 * j + 3])));
-          if (slab == BN / 64 - 1) {
+          if (slab == 1) {
             __syncwarp();
             if (lane == 0) {
               __threadfence();
@@ -1064,18 +1163,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
             r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v.w);
           }
         }
-        const int col0 = n_idx * 256 + slab * 64;
+        const int col0 = colw + slab * 64;
         if (row0 >= a.M || col0 >= a.N) continue;                     // nothing of this slab exists (warp-uniform)
-        unsigned char* cbuf = ebuf + (has_act ? 0u : (nstore & 1u)) * kEpiSlabBytes;
-        unsigned char* gbuf = ebuf + kEpiSlabBytes;
-        ++nstore;
-        // the copy engine must have finished reading the piece that is about to be rewritten:
-        // with two alternating pieces that is the store before the previous one
-        if (lane == 0) {
-          if (has_act) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        }
-        __syncwarp();
         if (a.gelu_grad_of != nullptr && row0 + lane < a.M) {
           // result *= gelu'(u[row, col]): this thread's 64 columns of u are 128 contiguous bytes
           const __nv_bfloat16* urow = reinterpret_cast<const __nv_bfloat16*>(a.gelu_grad_of) + (size_t)(row0 + lane) * a.N + col0;
@@ -1093,33 +1182,34 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
             }
           }
         }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          if (bias != nullptr && col0 + c * 8 < a.N) {
-            const uint4 qv = __ldg(reinterpret_cast<const uint4*>(bias + col0 + c * 8));     // N % 8 == 0: whole and aligned
-            const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              b[2 * e] = __uint_as_float(qw[e] << 16);
-              b[2 * e + 1] = __uint_as_float(qw[e] & 0xffff0000u);
-            }
-          }
-          const uint32_t off = (uint32_t)lane * 128u + (((uint32_t)c ^ sw) << 4);
-          uint4 g;
-          if (has_act) {
-            *reinterpret_cast<uint4*>(cbuf + off) = pack8<true>(r + c * 8, b, &g);
-            *reinterpret_cast<uint4*>(gbuf + off) = g;
-          } else {
-            *reinterpret_cast<uint4*>(cbuf + off) = pack8<false>(r + c * 8, b, &g);
-          }
+        // the copy engine must have finished reading this warp's piece before it is rewritten
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if (bias != nullptr) *(reinterpret_cast<uint32_t*>(bias_s) + lane) = slab == 0 ? bias_q[0] : bias_q[1];
+        __syncwarp();
+        if (has_act) {
+          if (bias != nullptr) slab_to_smem<true, true>(r, buf, bias_s, lane);
+          else slab_to_smem<false, true>(r, buf, bias_s, lane);
+        } else if (bias != nullptr) {
+          slab_to_smem<true, false>(r, buf, bias_s, lane);
+        } else {
+          slab_to_smem<false, false>(r, buf, bias_s, lane);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes, async-proxy read
         __syncwarp();
         if (lane == 0) {
-          tma_store_2d(&tmC, cbuf, col0, row0);
-          if (has_act) tma_store_2d(&tmAct, gbuf, col0, row0);
+          tma_store_2d(&tmC, buf, col0, row0);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        if (has_act) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+          slab_gelu_to_smem(r, buf, lane);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tmAct, buf, col0, row0);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
         }
       }
     }
@@ -1129,9 +1219,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       *abort_flag = 1;
     }
   }
+  // The peer may still be reading this CTA's shared memory or signalling it.  In a launch that went well the tails
+  // above have seen all its signals; after a wait that ran out a fence stands in for them.
+  if (*abort_flag != 0) asm volatile("fence.acq_rel.cluster;" ::: "memory");
   tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();                       // the peer may still be reading this CTA's shared memory or signalling it
+  __syncwarp();
+  cluster_arrive_relaxed();
+  cluster_wait();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -1210,7 +1304,7 @@ cudaError_t launch_pair(const CUtensorMap& mA, const CUtensorMap& mW, const CUte
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  gemm_sm100_2cta_kernel<A_MN, B_MN, WIDE><<<grid, kGemmThreads, kGemm2Smem, stream>>>(mA, mW, mOwn, mC, mAct, a);
+  gemm_sm100_2cta_kernel<A_MN, B_MN, WIDE><<<grid, kGemm2Threads, kGemm2Smem, stream>>>(mA, mW, mOwn, mC, mAct, a);
   return cudaGetLastError();
 }
 
@@ -1221,6 +1315,7 @@ int gemm_sk_tiles(int M, int N, int K, int sm_count) {
   const long long T = (long long)((M + 255) / 256) * ((N + 255) / 256);
   const int nkb = (K + BK - 1) / BK;
   if (G < 2 || nkb < 8 || T <= 0 || T > (1 << 30)) return 0;
+  if (2ll * G * nkb * (G + 1) >= (1ll << 31)) return 0;              // the kernel counts the split sequence in 32 bits
   const int R = (int)(T % G);
   if (R == 0) return 0;
   const long long rounds = (T + G - 1) / G;

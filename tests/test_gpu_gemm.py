@@ -60,6 +60,25 @@ def test_gemm_with_gelu_epilogue(shape, two_cta):
     assert float((g.float() - ref_g).norm() / ref_g.norm()) < 4e-3
 
 
+@pytest.mark.parametrize("N", [8, 64, 72, 128, 136, 200, 264])
+def test_epilogue_column_halves(N):
+    """Every epilogue warp owns half of a tile's columns in slabs of 64: outputs that end inside, at and just
+    behind a slab and a half, on several tiles per CTA pair, with bias, and with the second output."""
+    import pccl
+
+    M, K = 256 * 80 + 40, 72
+    A, W, bias = rnd((M, K), 21), rnd((N, K), 22, 0.1), rnd((N,), 23)
+    ref = A.float() @ W.float().t() + bias.float()
+    y, err = pccl._C.gemm(A, W, bias, None, True)
+    u, g, err2 = pccl._C.gemm_gelu(A, W, bias, True)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and int(err2.item()) == 0
+    check_close(y, ref, K)
+    assert torch.equal(u, y)
+    ref_g = torch.nn.functional.gelu(u.float(), approximate="tanh")
+    assert float((g.float() - ref_g).abs().max()) <= 1e-2 * float(ref_g.abs().max()) + 1e-3
+
+
 def test_linear_wrapper_and_identity():
     from pccl.ops.gemm import linear
 
