@@ -83,6 +83,9 @@ struct GemmArgs {
   // their W half in shared memory (three quarters of the operand bytes per FLOP from L2; both TMEM
   // accumulators belong to one unit).  Ignored with sk_tiles, panel flags or M <= 256.
   int wide;
+  // Plain CTA-pair products only: run as one 128 x tile_n tile per CTA with the contraction split over clusters of
+  // tile_split CTAs (see gemm_pick_tile).  0: the CTA-pair kernel.
+  int tile_n, tile_split;
 };
 
 // Bytes of sk_scratch / words of sk_flags needed for `pairs` CTA pairs.
@@ -92,6 +95,9 @@ constexpr size_t kGemmSkFlagsPerPair = 16;
 // How many leading tiles launch_gemm_sm100 would split along K for this shape on `sm_count` SMs
 // (0: none).  The caller provides scratch for sm_count / 2 pairs when this is non-zero.
 int gemm_sk_tiles(int M, int N, int K, int sm_count);
+
+// Width and split of the one-tile-per-CTA form for this shape, or 0 and 0 where the CTA-pair kernel is the faster one.
+void gemm_pick_tile(int M, int N, int K, int sm_count, int* tile_n, int* tile_split);
 
 // Launches on `stream`.  Returns cudaErrorInvalidValue for shapes the kernel does not take.
 cudaError_t launch_gemm_sm100(const GemmArgs& a, int sm_count, cudaStream_t stream);

@@ -53,6 +53,7 @@ struct SkWorkspace {
 };
 bool g_split_last_wave = true;
 bool g_split_single_round = false;        // also split shapes with fewer tiles than CTA pairs (slower back to back: measured)
+bool g_tiles = true;           // one tile per CTA where it is the faster form
 bool g_dynamic_tiles = false;  // hand tiles out at run time instead of dealing them out in advance
 int g_max_pairs = 0, g_group_m = 0;      // tuning knobs, 0: the kernel's defaults
 int g_wide = -1;                         // units of two row-tiles that share their W half: 1 always, 0 never, -1 where measured faster
@@ -77,6 +78,14 @@ SkWorkspace& sk_workspace(int device, cudaStream_t stream, int pairs) {
 void maybe_split_last_wave(GemmArgs& a, int device, cudaStream_t stream) {
   a.max_pairs = g_max_pairs;
   a.group_m = g_group_m;
+  if (g_tiles && a.two_cta && a.panel_flags == nullptr && !g_dynamic_tiles && g_max_pairs == 0 && g_wide <= 0 && !g_split_single_round &&
+      (reinterpret_cast<uintptr_t>(a.bias) & 15u) == 0) {
+    // too few 256 x 256 tiles to occupy the device: one smaller tile per CTA, its contraction split over a cluster.
+    // Not where tiles are handed out at run time (SMs are then held by collectives), nor beside the settings that
+    // force another form.
+    gemm_pick_tile(a.M, a.N, a.K, sm_count(device), &a.tile_n, &a.tile_split);
+    if (a.tile_n > 0) return;
+  }
   if (g_wide != 0 && g_max_pairs == 0 && a.two_cta && a.panel_flags == nullptr && a.M > 256) {
     // Units of two row-tiles (never split along K).  Measured on the training shapes: 6-28 % faster than
     // single tiles for contractions of 4096 and more when the units fill their rounds, slower for short
@@ -449,6 +458,12 @@ void bind_gemm(py::module_& m) {
   m.def("gemm_set_dynamic_tiles", [](bool on) { g_dynamic_tiles = on; }, py::arg("on"),
         "CTA pairs draw their tiles from a counter at run time (robust beside kernels that hold some SMs) instead of a "
         "fixed round-robin share; excludes the split of the last round");
+  m.def("gemm_set_tiles", [](bool on) { g_tiles = on; }, "allow the one-tile-per-CTA form (default on)");
+  m.def("gemm_pick_tile", [](int M, int N, int K, int sms) {
+    int n = 0, s = 0;
+    gemm_pick_tile(M, N, K, sms, &n, &s);
+    return std::make_tuple(n, s);
+  }, "(tile width, split) of the one-tile-per-CTA form for a shape; (0, 0): the CTA-pair kernel");
   m.def("gemm_set_split_last_wave", [](bool on, bool single_round) { g_split_last_wave = on; g_split_single_round = single_round; },
         py::arg("on"), py::arg("single_round") = false,
         "split the tiles of a partly filled last round along K over all CTA pairs (default on); single_round: also "

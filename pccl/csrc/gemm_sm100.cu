@@ -1234,6 +1234,254 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
   }
 }
 
+// ---------------------------------------------------------------- one tile per CTA, contraction split over a cluster
+// For products whose 256 x 256 tiles are too few to occupy the device (see gemm_pick_tile): one CTA works on
+// one tile of 128 rows, and a cluster of `split` CTAs shares the contraction of a tile, so that small outputs still
+// reach every SM.  Such a launch is a chain of latencies, and everything here shortens that chain: no persistence and
+// no scheduling; the first loads leave before the block has met for the first time; two CTAs of the narrow form fit on an SM
+// (96 KiB, 128 TMEM columns), so one's start and end hide behind the other's main loop; all eight warps drain the accumulator.
+// The partial sums of a cluster meet in shared memory: each CTA leaves its fp32 tile in its own (the stages are
+// free by then) and adds up one column slice of all of them through distributed shared memory, in rank order.  No
+// global scratch, no flags: nothing is shared between launches.
+// Two widths: 128 columns, two CTAs per SM; 256 columns, one CTA per SM with twice the work per MMA, for split long
+// contractions.  Figures at gemm_pick_tile.
+constexpr int kTileThreads = 256;
+template <int TN>
+struct TileCfg {
+  static constexpr int kStages = TN == 128 ? 3 : 4;
+  static constexpr int kPerSm = TN == 128 ? 2 : 1;                               // CTAs per SM
+  static constexpr uint32_t kStage = kHalfBytes + TN * BK * 2;                     // 128 rows of A, TN rows of W
+  static constexpr uint32_t kBarOff = kStages * kStage;
+  static constexpr uint32_t kSmem = kBarOff + 128 + 1024;
+  static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+  static_assert(128 * TN * 4 <= kBarOff, "the fp32 tile must fit into the stages");
+};
+
+struct TileArgs {
+  int M, N, K, split, tiles_n;
+  void* C;
+  const void* bias;
+  void* act_out;
+  const void* gelu_grad_of;
+  int* error;
+};
+
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_u32(smem_dst)),
+      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void mma_bf16_tile(uint32_t tmem_d, uint32_t da_lo, uint32_t db_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 da, {%1, %5};\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(da_lo), "r"(db_lo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
+      : "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+
+// This CTA's column slice of the tile: TN / 8 / SPLIT chunks of eight columns per row, summed over the cluster.
+// The fp32 tile lies in shared memory as rows of TN / 4 four-float pieces, piece c of row r at c ^ (r % 32).
+template <int SPLIT, int TN>
+__device__ __forceinline__ void tile_reduce_store(const TileArgs& a, uint32_t tile_smem, int rank, int m0, int n0) {
+  constexpr int CPR = TN / 8 / SPLIT;
+  uint32_t base[SPLIT];
+#pragma unroll
+  for (int p = 0; p < SPLIT; ++p) base[p] = SPLIT == 1 ? tile_smem : map_to_cta(tile_smem, (uint32_t)p);
+#pragma unroll 2
+  for (int i = threadIdx.x; i < 128 * CPR; i += kTileThreads) {
+    const int row = i / CPR, ch = rank * CPR + i % CPR;
+    const int gr = m0 + row, gc = n0 + ch * 8;
+    if (gr >= a.M || gc >= a.N) continue;                    // N % 8 == 0: a chunk is inside or outside as a whole
+    const size_t off = (size_t)gr * a.N + gc;
+    uint4 bq = make_uint4(0u, 0u, 0u, 0u), uq = make_uint4(0u, 0u, 0u, 0u);
+    if (a.bias != nullptr) bq = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.bias) + gc));
+    if (a.gelu_grad_of != nullptr) uq = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.gelu_grad_of) + off));
+    const uint32_t o0 = (uint32_t)(row * (TN * 4) + (((2 * ch) ^ (row & 31)) << 4)), o1 = (uint32_t)(row * (TN * 4) + (((2 * ch + 1) ^ (row & 31)) << 4));
+    float4 v0[SPLIT], v1[SPLIT];
+#pragma unroll
+    for (int p = 0; p < SPLIT; ++p) {
+      v0[p] = ld_cluster_f4(base[p] + o0);
+      v1[p] = ld_cluster_f4(base[p] + o1);
+    }
+    float f[8] = {v0[0].x, v0[0].y, v0[0].z, v0[0].w, v1[0].x, v1[0].y, v1[0].z, v1[0].w};
+#pragma unroll
+    for (int p = 1; p < SPLIT; ++p) {
+      f[0] += v0[p].x, f[1] += v0[p].y, f[2] += v0[p].z, f[3] += v0[p].w;
+      f[4] += v1[p].x, f[5] += v1[p].y, f[6] += v1[p].z, f[7] += v1[p].w;
+    }
+    const uint32_t bw[4] = {bq.x, bq.y, bq.z, bq.w}, uw[4] = {uq.x, uq.y, uq.z, uq.w};
+    uint32_t w[4], g[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float x0 = f[2 * e] + __uint_as_float(bw[e] << 16), x1 = f[2 * e + 1] + __uint_as_float(bw[e] & 0xffff0000u);
+      if (a.gelu_grad_of != nullptr) {
+        x0 *= gelu_tanh_grad(__uint_as_float(uw[e] << 16));
+        x1 *= gelu_tanh_grad(__uint_as_float(uw[e] & 0xffff0000u));
+      }
+      const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+      w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      if (a.act_out != nullptr) {
+        const __nv_bfloat162 hg = __floats2bfloat162_rn(gelu_tanh(__low2float(h)), gelu_tanh(__high2float(h)));
+        g[e] = *reinterpret_cast<const uint32_t*>(&hg);
+      }
+    }
+    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.C) + off) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (a.act_out != nullptr) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.act_out) + off) = make_uint4(g[0], g[1], g[2], g[3]);
+  }
+}
+
+template <bool A_MN, bool B_MN, int TN>
+__global__ void __launch_bounds__(kTileThreads, TileCfg<TN>::kPerSm)
+    gemm_sm100_tile_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
+                           const __grid_constant__ TileArgs a) {
+  using Cfg = TileCfg<TN>;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::kBarOff);
+  uint64_t* empty = full + Cfg::kStages;
+  uint64_t* done = empty + Cfg::kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int rank = (int)blockIdx.x % a.split, tile = (int)blockIdx.x / a.split;
+  const int m_idx = tile / a.tiles_n;
+  const int m0 = m_idx * 128, n0 = (tile - m_idx * a.tiles_n) * TN;
+  const int nkb = (a.K + BK - 1) / BK;
+  const int kb0 = nkb * rank / a.split, n = nkb * (rank + 1) / a.split - kb0;      // this CTA's k-blocks
+  bool ok = true;
+
+  auto load = [&](int i, int s) {
+    unsigned char* sa = smem + (size_t)s * Cfg::kStage;
+    mbar_expect_tx(full + s, Cfg::kStage);
+    const int k = (kb0 + i) * BK;
+    if (A_MN) tma_load_3d(sa, &tmA, 0, k, m0 >> 6, full + s);
+    else tma_load_2d(sa, &tmA, k, m0, full + s);
+#pragma unroll
+    for (int h = 0; h < TN / 128; ++h) {
+      if (B_MN) tma_load_3d(sa + (1 + h) * kHalfBytes, &tmW, 0, k, (n0 >> 6) + 2 * h, full + s);
+      else tma_load_2d(sa + (1 + h) * kHalfBytes, &tmW, k, n0 + 128 * h, full + s);
+    }
+  };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < Cfg::kStages; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    fence_proxy_async_smem();
+    for (int i = 0; i < n && i < Cfg::kStages; ++i) load(i, i);      // the barriers they signal are this thread's own
+  } else if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)TN)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0 && lane == 0) {
+    int s = 0;
+    uint32_t ph = 0;
+    for (int i = Cfg::kStages; i < n; ++i) {
+      if (!gemm_wait(empty + s, ph, abort_flag)) {
+        atomicCAS(a.error, 0, kErrProducer);
+        *abort_flag = 1;
+        break;
+      }
+      load(i, s);
+      if (++s == Cfg::kStages) {
+        s = 0;
+        ph ^= 1u;
+      }
+    }
+  } else if (warp == 1 && lane == 0) {
+    constexpr uint32_t idesc = Cfg::kIdesc | (A_MN ? (1u << 15) : 0u) | (B_MN ? (1u << 16) : 0u);
+    constexpr uint32_t a_step = A_MN ? (2048 >> 4) : (32 >> 4);
+    constexpr uint32_t b_step = B_MN ? (2048 >> 4) : (32 >> 4);
+    const uint32_t da0 = desc_lo(smem_u32(smem), A_MN);
+    const uint32_t db0 = desc_lo(smem_u32(smem) + kHalfBytes, B_MN);
+    uint32_t s = 0, ph = 0;
+    for (int i = 0; i < n; ++i) {
+      if (!gemm_wait(full + s, ph, abort_flag)) {
+        ok = false;
+        atomicCAS(a.error, 0, kErrMma);
+        *abort_flag = 1;
+        break;
+      }
+      const uint32_t da = da0 + s * (Cfg::kStage >> 4), db = db0 + s * (Cfg::kStage >> 4);
+#pragma unroll
+      for (int k = 0; k < BK / 16; ++k) mma_bf16_tile(tmem_base, da + k * a_step, db + k * b_step, idesc, (i > 0 || k > 0) ? 1u : 0u);
+      mma_commit(empty + s);
+      if (++s == (uint32_t)Cfg::kStages) {
+        s = 0;
+        ph ^= 1u;
+      }
+    }
+    if (ok) mma_commit(done);
+  }
+  __syncwarp();
+
+  // ---- the accumulator, to shared memory as fp32.  All MMAs have read their stages by then.
+  if (lane == 0) ok = gemm_wait(done, 0u, abort_flag);
+  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+  if (ok) {
+    tc_fence_after();
+    const int row = (warp & 3) * 32 + lane, half = warp >> 2;            // TN / 2 columns each
+    unsigned char* dst = smem + row * (TN * 4);
+#pragma unroll 1
+    for (int c0 = half * (TN / 2); c0 < (half + 1) * (TN / 2); c0 += 64) {
+      uint32_t r[64];
+      const uint32_t taddr = tmem_base + (uint32_t)c0 + ((uint32_t)((warp & 3) * 32) << 16);
+      tmem_ld32(taddr, r);
+      tmem_ld32(taddr + 32, r + 32);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        *reinterpret_cast<uint4*>(dst + (((c0 / 4 + j) ^ lane) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+    }
+  } else if (lane == 0) {
+    atomicCAS(a.error, 0, kErrEpilogue);
+    *abort_flag = 1;
+  }
+  tc_fence_before();
+  __syncwarp();
+  if (a.split > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TN) : "memory");
+  }
+  const uint32_t tile_smem = smem_u32(smem);
+  if (a.split == 1) {
+    tile_reduce_store<1, TN>(a, tile_smem, rank, m0, n0);
+    return;
+  }
+  if (a.split == 2) tile_reduce_store<2, TN>(a, tile_smem, rank, m0, n0);
+  else if (a.split == 4) tile_reduce_store<4, TN>(a, tile_smem, rank, m0, n0);
+  else tile_reduce_store<8, TN>(a, tile_smem, rank, m0, n0);
+  __syncwarp();
+  cluster_arrive_relaxed();                 // nobody leaves while its tile is still being read
+  cluster_wait();
+}
+
 // ---------------------------------------------------------------- host side
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1310,7 +1558,84 @@ cudaError_t launch_pair(const CUtensorMap& mA, const CUtensorMap& mW, const CUte
   return cudaGetLastError();
 }
 
+template <bool A_MN, bool B_MN, int TN>
+cudaError_t launch_tile_form(const CUtensorMap& mA, const CUtensorMap& mW, const TileArgs& ta, int tiles, cudaStream_t stream) {
+  static thread_local bool configured[64] = {false};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    e = cudaFuncSetAttribute(gemm_sm100_tile_kernel<A_MN, B_MN, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TileCfg<TN>::kSmem);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * ta.split));
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.dynamicSmemBytes = TileCfg<TN>::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ta.split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, gemm_sm100_tile_kernel<A_MN, B_MN, TN>, mA, mW, ta);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <int TN>
+cudaError_t launch_tile(const CUtensorMap& mA, const CUtensorMap& mW, const GemmArgs& a, int split, cudaStream_t stream) {
+  TileArgs ta;
+  ta.M = a.M, ta.N = a.N, ta.K = a.K, ta.split = split, ta.tiles_n = (a.N + TN - 1) / TN;
+  ta.C = a.C, ta.bias = a.bias, ta.act_out = a.act_out, ta.gelu_grad_of = a.gelu_grad_of, ta.error = a.error;
+  const int tiles = ((a.M + 127) / 128) * ta.tiles_n;
+  if (a.a_mn && a.b_mn) return launch_tile_form<true, true, TN>(mA, mW, ta, tiles, stream);
+  if (a.a_mn) return launch_tile_form<true, false, TN>(mA, mW, ta, tiles, stream);
+  if (a.b_mn) return launch_tile_form<false, true, TN>(mA, mW, ta, tiles, stream);
+  return launch_tile_form<false, false, TN>(mA, mW, ta, tiles, stream);
+}
+
 }  // namespace
+
+// Which form of the one-tile-per-CTA kernel, if any, is expected to beat the CTA-pair kernel.  Only products of at
+// most one round of 256 x 256 tiles come into question.  The estimates (ns) are fits of kernel times measured for
+// outputs of 64 x 256 to 4096 x 1024 and contractions of 128 to 8192 (checked up to 50304): a fixed part, a part
+// per k-block, and for a split the exchange of partial sums (loads from another SM's shared memory are slow: two CTAs
+// spend 1.6 us on it, four 3 us, and all of them together move about 2.2 TB/s).
+//   pair 256 x 256           5900 + 281 per k-block
+//   one CTA, 128 columns     4100 + 265 per k-block while the CTAs have an SM each, else 5400 + 400
+//   one CTA, 256 columns     5700 + 285 per k-block, an SM each; worth it only for split long contractions
+// Measured on both sides of the line (us, pair / chosen): 256 x 768 x 256 6.8 / 5.1; 1000 x 1024 x 3072 19.7 / 13.7;
+// 1024 x 2048 x 4096 25.1 / 20.4; 2048 x 1024 x 50304 228 / 157; pair kept: 1000 x 3072 x 1024 10.9 (against 11.3),
+// 4096 x 1024 x 2048 16.2 (16.9).
+void gemm_pick_tile(int M, int N, int K, int sm_count, int* tile_n, int* tile_split) {
+  *tile_n = 0;
+  *tile_split = 0;
+  const long long nkb = (K + BK - 1) / BK;
+  const long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  if (pair_tiles > sm_count / 2) return;
+  long long best = 5900 + 281 * nkb;
+  for (int tn = 128; tn <= 256; tn += 128) {
+    const long long t = (long long)((M + 127) / 128) * ((N + tn - 1) / tn);
+    for (int s = tn == 128 ? 1 : 2; s <= 8; s *= 2) {
+      const long long ctas = t * s;
+      if (s > 1 && nkb < 2 * s) break;
+      if (ctas > (tn == 128 ? 2 : 1) * (long long)sm_count) break;
+      if (s == 8 && (tn == 256 || ctas > 96)) break;                    // clusters of eight are placed slowly: 2-3 times slower beyond
+      const bool alone = ctas <= sm_count;
+      const long long kb = (nkb + s - 1) / s;
+      long long cost = tn == 256 ? 5700 + 285 * kb : (alone ? 4100 + 265 * kb : 5400 + 400 * kb);
+      if (s == 1 && nkb >= 64) cost += 66 * kb;                         // long rows read by all CTAs in step: a quarter slower
+      if (s > 1) cost += tn == 256 ? (s == 2 ? 2700 + 10 * t : 4800 + 50 * t) : (s == 2 ? 1600 : s == 4 ? 3000 : 5500) + 12 * t * (s - 1);
+      if (cost < best) {
+        best = cost;
+        *tile_n = tn;
+        *tile_split = s;
+      }
+    }
+  }
+}
 
 int gemm_sk_tiles(int M, int N, int K, int sm_count) {
   const int G = sm_count / 2;
@@ -1358,6 +1683,13 @@ cudaError_t launch_gemm_sm100(const GemmArgs& a_in, int sm_count, cudaStream_t s
     if (!okA || !okW) return cudaErrorInvalidValue;
     if (a.b_mn) mOwn = mW;
     else if (!make_map(&mOwn, own, own_rows, (uint64_t)a.K, 128)) return cudaErrorInvalidValue;
+    if (a.tile_n > 0) {
+      if (fused || a.sk_tiles > 0 || a.sched_counter != nullptr || (a.tile_n != 128 && a.tile_n != 256)) return cudaErrorInvalidValue;
+      const int s = a.tile_split;
+      if ((s != 1 && s != 2 && s != 4 && s != 8) || s > (a.K + BK - 1) / BK) return cudaErrorInvalidValue;   // every CTA needs a k-block
+      if (a.bias != nullptr && (reinterpret_cast<uintptr_t>(a.bias) & 15u)) return cudaErrorInvalidValue;
+      return a.tile_n == 128 ? launch_tile<128>(mA, mW, a, s, stream) : launch_tile<256>(mA, mW, a, s, stream);
+    }
     if (!make_map_store(&mC, a.C, (uint64_t)a.M, (uint64_t)a.N)) return cudaErrorInvalidValue;
     if (a.act_out != nullptr) {
       if (!make_map_store(&mAct, a.act_out, (uint64_t)a.M, (uint64_t)a.N)) return cudaErrorInvalidValue;

@@ -79,6 +79,50 @@ def test_epilogue_column_halves(N):
     assert float((g.float() - ref_g).abs().max()) <= 1e-2 * float(ref_g.abs().max()) + 1e-3
 
 
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("shape", [(8, 64, 8), (64, 64, 64), (128, 128, 128), (136, 192, 200), (320, 320, 1032), (64, 256, 8192),
+                                   (256, 256, 2048), (1000, 1024, 3072), (1024, 2048, 4096), (512, 1024, 9000)])
+def test_one_tile_per_cta(shape, layout):
+    """Small outputs: one 128-row tile per CTA, the contraction split over clusters of 1, 2, 4 or 8 CTAs; edges of
+    tiles in every direction, a K that ends inside a k-block, bias, activation and gelu' factor."""
+    import pccl
+    from pccl.ops.gemm import check_errors
+
+    C = pccl._C
+    M, N, K = shape
+    if layout == "tn" and M % 64:
+        M = (M + 63) // 64 * 64
+    tile, split = C.gemm_pick_tile(M, N, K, 148)
+    assert tile in (128, 256) and split in (1, 2, 4, 8)
+    x, w, bias = rnd((M, K), 31), rnd((N, K), 32, 0.05), rnd((N,), 33)
+    ref = x.float() @ w.float().t()
+    a = x.t().contiguous() if layout == "tn" else x
+    b = w if layout == "nt" else w.t().contiguous()
+    flags = (layout == "tn", layout != "nt")
+    y = C.gemm_ex(a, b, *flags, bias, None, None)
+    check_close(y, ref + bias.float(), K)
+    u = rnd((M, N), 34)
+    ur = u.float().requires_grad_()
+    (grad,) = torch.autograd.grad(torch.nn.functional.gelu(ur, approximate="tanh").sum(), ur)
+    check_close(C.gemm_ex(a, b, *flags, None, None, u), ref * grad, K)
+    if layout == "nt":
+        v, g, _ = C.gemm_gelu(x, w, bias, True)
+        assert torch.equal(v, y)
+        ref_g = torch.nn.functional.gelu(v.float(), approximate="tanh")
+        assert float((g.float() - ref_g).abs().max()) <= 1e-2 * float(ref_g.abs().max()) + 1e-3
+    # the fp32 sums of a split are added in a fixed order: the same twice
+    assert torch.equal(y, C.gemm_ex(a, b, *flags, bias, None, None))
+    check_errors()
+    # and the CTA-pair kernel agrees to the rounding of the result
+    C.gemm_set_tiles(False)
+    try:
+        z = C.gemm_ex(a, b, *flags, bias, None, None)
+    finally:
+        C.gemm_set_tiles(True)
+    assert float((y.float() - z.float()).norm() / z.float().norm()) < 2e-3
+    assert C.gemm_pick_tile(8192, 8192, 2048, 148) == (0, 0)
+
+
 def test_linear_wrapper_and_identity():
     from pccl.ops.gemm import linear
 
