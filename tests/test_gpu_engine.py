@@ -83,6 +83,43 @@ def test_cross_entropy_forward_backward():
     torch.testing.assert_close(small.float(), r2.grad, rtol=2e-2, atol=1e-6)
 
 
+@pytest.mark.parametrize("rows,vocab", [(1, 8), (3, 13), (5, 1023), (700, 4099), (1500, 4096), (301, 16384), (299, 50304), (2, 102400)])
+def test_cross_entropy_rows_per_block_and_ragged_columns(rows, vocab):
+    """Blocks walk over several rows and take the next one in while they finish the last: more rows than blocks and
+    fewer, each block size, columns past the last whole vector, a row stride above the row, large and masked logits."""
+    import pccl
+
+    g = torch.Generator(device="cuda:0").manual_seed(rows + vocab)
+    stride = (vocab + 7) // 8 * 8 + 8
+    store = torch.full((rows, stride), 7.0, device="cuda:0", dtype=torch.bfloat16)
+    logits = store[:, :vocab]
+    logits.copy_(torch.randn(rows, vocab, generator=g, device="cuda:0") * 4 + 50 * torch.randn(rows, 1, generator=g, device="cuda:0"))
+    if vocab > 8:
+        logits[:, ::5] = float("-inf")                     # masked columns
+    targets = torch.randint(0, vocab, (rows,), generator=g, device="cuda:0")
+    targets = torch.where((targets % 5 == 0) & (targets + 1 < vocab), targets + 1, targets)
+    if rows > 1:
+        targets[1] = -100
+    ref = logits.double()
+    keep = targets != -100
+    lse = torch.logsumexp(ref, -1)
+    picked = ref.gather(1, targets.clamp(min=0).unsqueeze(1)).squeeze(1)
+    grad = torch.softmax(ref, -1)
+    grad[torch.arange(rows), targets.clamp(min=0)] -= 1.0
+    grad = torch.where(keep.unsqueeze(1), grad, torch.zeros_like(grad)) * 0.25
+    loss = torch.zeros(1, device="cuda:0")
+    bad = torch.zeros(1, dtype=torch.int32, device="cuda:0")
+    pccl._C.ce_fwd_bwd(logits, targets, loss, 0.25, -100, bad)
+    want = float((lse - picked)[keep].sum())
+    assert int(bad) == 0
+    if want == want and abs(want) != float("inf"):
+        assert abs(float(loss) - want) <= 2e-5 * max(1.0, abs(want))
+        # one bf16 rounding of each gradient, fp32 exponentials in front of it
+        assert float((logits.double() - grad).abs().max()) <= 2.0 ** -8 * 0.25
+        assert float((logits.double() - grad).norm() / grad.norm()) < 3e-3
+    assert bool((store[:, vocab:] == 7.0).all())
+
+
 def test_cross_entropy_reports_targets_outside_the_vocabulary():
     """A label that is neither a class nor the ignore index must not be used as an index: its row
     is left out (zero loss, zero gradient) and counted in the error word."""
