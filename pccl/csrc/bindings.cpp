@@ -329,6 +329,7 @@ void reduce_scatter(Comm& c, int gid, std::vector<at::Tensor> outs, std::vector<
     const uint64_t len = std::min(cap, n - e0);
     a.stage_off = c.staging_off();
     a.sub_elems = len;
+    a.stage_elems = (len + 7) / 8 * 8;               // cap is a multiple of 8, so the padded blocks fit as well
     for (int i = 0; i < l.n; ++i) {
       a.in[i] = (const char*)ins[i].data_ptr() + e0 * si;
       a.out[i] = (char*)outs[i].data_ptr() + e0 * so;
@@ -408,6 +409,7 @@ void all_reduce(Comm& c, int gid, std::vector<at::Tensor> ts, int algo, int nlan
       a.rs.out_sub_stride = blk * s;
       a.rs.stage_off = c.staging_off();
       a.rs.sub_elems = len;
+      a.rs.stage_elems = (len + 7) / 8 * 8;          // cap is a multiple of 8
       a.ag.nsub = 1;
       a.ag.sub_bytes = len * s;
       a.ag.in_sub_stride = blk * s;

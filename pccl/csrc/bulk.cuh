@@ -80,12 +80,14 @@ struct BulkPipe {
   uint64_t* full;    // kBulkStages mbarriers
   uint32_t count;    // chunks pushed through the ring so far (stage = count % N, parity = (count / N) & 1)
   uint64_t timeout_ns;
+  bool dirty;        // copy-engine stores were issued since the last flush
 };
 
 __device__ __forceinline__ void bulk_pipe_init(BulkPipe& p, unsigned char* smem, uint64_t timeout_ns) {
   p.stages = reinterpret_cast<char*>(smem);
   p.full = reinterpret_cast<uint64_t*>(smem + (size_t)kBulkStageBytes * kBulkStages);
   p.count = 0;
+  p.dirty = false;
   p.timeout_ns = timeout_ns;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kBulkStages; ++i) mbar_init(p.full + i, 1);
@@ -137,14 +139,18 @@ __device__ __forceinline__ bool cta_bulk_copy(BulkPipe& p, char* const* dsts, in
     s_bulk_ok = ok ? 1 : 0;
   }
   p.count += nchunks;
+  p.dirty = true;
   __syncthreads();
   const int ok = s_bulk_ok;
   __syncthreads();
   return ok != 0;
 }
 
-// Wait until every store issued by this CTA has been performed (then a release flag may follow).
-__device__ __forceinline__ void cta_bulk_flush() {
+// Wait until every copy-engine store issued by this CTA has been performed (then a release flag may follow).  Costs a
+// system-scope fence, so messages that went through the thread loops only skip it.
+__device__ __forceinline__ void cta_bulk_flush(BulkPipe& p) {
+  if (!p.dirty) return;                         // the same for all threads
+  p.dirty = false;
   if (threadIdx.x == 0) {
     bulk_wait_all();
     asm volatile("fence.proxy.async;" ::: "memory");   // async-proxy writes before the generic-proxy flag

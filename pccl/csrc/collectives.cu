@@ -33,7 +33,7 @@ __device__ __forceinline__ int step_kind(int algo, int t) { return kSlotStep0 + 
 constexpr uint64_t kBulkMinBytes = 192 * 1024;
 
 // Copy one range to ndst destinations: copy engine when aligned, thread loops otherwise.
-template <bool REMOTE_SRC>
+template <bool REMOTE_SRC, bool RAGGED = true>
 __device__ __forceinline__ bool lane_copy(BulkPipe& pipe, char* const* dsts, int ndst, const char* src, uint64_t len) {
   if (len == 0 || ndst == 0) return true;
   bool aligned = (reinterpret_cast<uintptr_t>(src) & 15u) == 0 && len >= kBulkMinBytes;
@@ -48,24 +48,24 @@ __device__ __forceinline__ bool lane_copy(BulkPipe& pipe, char* const* dsts, int
     int nr = 0;
     for (int d = 0; d < ndst; ++d)
       if (dsts[d] != src) rest[nr++] = dsts[d] + done;
-    cta_copy_multi<REMOTE_SRC>(rest, nr, src + done, len - done);
+    cta_copy_multi<REMOTE_SRC, RAGGED>(rest, nr, src + done, len - done);
   }
   return true;
 }
-template <bool REMOTE_SRC>
+template <bool REMOTE_SRC, bool RAGGED = true>
 __device__ __forceinline__ bool lane_copy1(BulkPipe& pipe, char* dst, const char* src, uint64_t len) {
   if (dst == src) return true;
   char* d[1] = {dst};
-  return lane_copy<REMOTE_SRC>(pipe, d, 1, src, len);
+  return lane_copy<REMOTE_SRC, RAGGED>(pipe, d, 1, src, len);
 }
 
 // Publish a flag after data: first make sure the copy engine's stores have been performed.
-__device__ __forceinline__ void publish_mask(const GroupDev& g, const LaneCtx& c, int kind, unsigned mask) {
-  cta_bulk_flush();
+__device__ __forceinline__ void publish_mask(BulkPipe& pipe, const GroupDev& g, const LaneCtx& c, int kind, unsigned mask) {
+  cta_bulk_flush(pipe);
   cta_signal_mask(g, c, kind, mask);
 }
-__device__ __forceinline__ void publish(const GroupDev& g, const LaneCtx& c, int kind, int dst) {
-  publish_mask(g, c, kind, 1u << dst);
+__device__ __forceinline__ void publish(BulkPipe& pipe, const GroupDev& g, const LaneCtx& c, int kind, int dst) {
+  publish_mask(pipe, g, c, kind, 1u << dst);
 }
 
 // ============================================================================ all-gather
@@ -104,7 +104,7 @@ __device__ __forceinline__ void all_gather_body(const AllGatherArgs& a, BulkPipe
       char* d = out != nullptr ? out + opos(0, j) : mine + pos(0, j);
       if (!lane_copy1<false>(pipe, d, own(j), len)) return;
     }
-    cta_bulk_flush();
+    cta_bulk_flush(pipe);
     return;
   }
 
@@ -115,7 +115,7 @@ __device__ __forceinline__ void all_gather_body(const AllGatherArgs& a, BulkPipe
       for (int j = 0; j < a.nsub; ++j)
         if (!lane_copy1<false>(pipe, stage + (uint64_t)j * a.in_sub_stride + lo, own(j), len)) return;
     }
-    publish_mask(g, c, kSlotEntry, others);
+    publish_mask(pipe, g, c, kSlotEntry, others);
     for (int j = 0; j < a.nsub; ++j) {
       char* d = out != nullptr ? out + opos(me, j) : mine + pos(me, j);
       if (!lane_copy1<false>(pipe, d, own(j), len)) return;
@@ -129,7 +129,7 @@ __device__ __forceinline__ void all_gather_body(const AllGatherArgs& a, BulkPipe
         if (!lane_copy1<true>(pipe, d, theirs + (uint64_t)j * a.in_sub_stride + lo, len)) return;
       }
     }
-    publish_mask(g, c, kSlotExit, others);     // flush: our loads of their memory are complete
+    publish_mask(pipe, g, c, kSlotExit, others);     // flush: our loads of their memory are complete
     cta_wait_mask(g, c, kSlotExit, others);
     return;
   }
@@ -173,14 +173,14 @@ __device__ __forceinline__ void all_gather_body(const AllGatherArgs& a, BulkPipe
       if (out != nullptr) dsts[nd++] = out + opos(me, j);
       if (!lane_copy<false>(pipe, dsts, nd, own(j), len)) return;
     }
-    publish_mask(g, c, kSlotStep0, others);
+    publish_mask(pipe, g, c, kSlotStep0, others);
     if (!cta_wait_mask(g, c, kSlotStep0, others)) return;
   } else {
     // Ring and recursive doubling: forward what has arrived.
     if (in != nullptr)
       for (int j = 0; j < a.nsub; ++j)
         if (!lane_copy1<false>(pipe, mine + pos(me, j), own(j), len)) return;
-    publish_mask(g, c, kSlotEntry, others);      // flush: later steps read the landing zone
+    publish_mask(pipe, g, c, kSlotEntry, others);      // flush: later steps read the landing zone
     unsigned entered = 0, arrived = 0;
     const int n = num_steps(algo, P);
     for (int t = 0; t < n; ++t) {
@@ -202,7 +202,7 @@ __device__ __forceinline__ void all_gather_body(const AllGatherArgs& a, BulkPipe
             if (!lane_copy1<true>(pipe, theirs + pos(b, j), mine + pos(b, j), len)) return;
           }
         }
-      publish(g, c, step_kind(algo, t), s.dst);
+      publish(pipe, g, c, step_kind(algo, t), s.dst);
     }
     for (int t = 0; t < n; ++t)
       if (!((arrived >> t) & 1u))
@@ -219,7 +219,7 @@ __device__ __forceinline__ void all_gather_body(const AllGatherArgs& a, BulkPipe
         }
       }
   }
-  cta_bulk_flush();
+  cta_bulk_flush(pipe);
 }
 
 __global__ void __launch_bounds__(kCollThreads, 1) all_gather_kernel(const __grid_constant__ AllGatherArgs a) {
@@ -230,13 +230,14 @@ __global__ void __launch_bounds__(kCollThreads, 1) all_gather_kernel(const __gri
 }
 
 // ============================================================================ reduce-scatter
-// Sum nsrc sources (first one of type TA, the rest TW) into one destination.
-template <int TA, int TW, int TOUT, bool REMOTE_W>
+// Sum nsrc sources (first one of type TA, the rest TW) into one destination.  RAGGED kernels have the code for
+// misaligned operands in the place of the copy-engine path (some operand of every sum is misaligned there).
+template <int TA, int TW, int TOUT, bool REMOTE_W, bool RAGGED>
 __device__ __forceinline__ bool lane_reduce(BulkPipe& pipe, char* out, const char* a_src, const char* const* w, int nw,
                                             uint64_t cnt, float scale) {
   constexpr uint64_t SA = Elem<TA>::size, SO = Elem<TOUT>::size;
   uint64_t done = 0;
-  if constexpr (TA == TW) {
+  if constexpr (TA == TW && !RAGGED) {
     bool aligned = cnt * SA >= kBulkMinBytes && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 &&
                    (reinterpret_cast<uintptr_t>(a_src) & 15u) == 0;
     for (int k = 0; k < nw; ++k) aligned = aligned && (reinterpret_cast<uintptr_t>(w[k]) & 15u) == 0;
@@ -254,12 +255,12 @@ __device__ __forceinline__ bool lane_reduce(BulkPipe& pipe, char* out, const cha
     const char* wt[kMaxReduceSrc];
     for (int k = 0; k < nw; ++k) wt[k] = w[k] + done * Elem<TW>::size;
     char* o = out + done * SO;
-    cta_reduce<TA, TW, TOUT, REMOTE_W>(&o, 1, a_src + done * SA, wt, nw, cnt - done, scale);
+    cta_reduce<TA, TW, TOUT, REMOTE_W, RAGGED>(&o, 1, a_src + done * SA, wt, nw, cnt - done, scale);
   }
   return true;
 }
 
-template <int TIN, int TW, int TOUT>
+template <int TIN, int TW, int TOUT, bool RAGGED>
 __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, BulkPipe& pipe, uint32_t coll) {
   const GroupDev& g = a.g;
   const int P = g.size;
@@ -280,13 +281,13 @@ __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, 
   };
   auto out_ptr = [&](int j) -> char* { return out + (uint64_t)j * a.out_sub_stride + lo * SO; };
   auto stage_ptr = [&](int rank, int slot, int j) -> char* {
-    return g.heap[rank] + a.stage_off + (((uint64_t)slot * a.nsub + j) * a.sub_elems + lo) * SW;
+    return g.heap[rank] + a.stage_off + (((uint64_t)slot * a.nsub + j) * a.stage_elems + lo) * SW;
   };
 
   if (P == 1) {
     for (int j = 0; j < a.nsub; ++j) {
       char* o = out_ptr(j);
-      cta_reduce<TIN, TIN, TOUT, false>(&o, 1, in_ptr(in, 0, j), nullptr, 0, cnt, a.scale);
+      cta_reduce<TIN, TIN, TOUT, false, RAGGED>(&o, 1, in_ptr(in, 0, j), nullptr, 0, cnt, a.scale);
     }
     return;
   }
@@ -299,7 +300,7 @@ __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, 
       const char* w[kMaxReduceSrc];
       int nw = 0;
       for (int k = 1; k < P; ++k) w[nw++] = in_ptr(g.heap[pmod(me + k, P)] + a.in_off, me, j);
-      if (!lane_reduce<TIN, TIN, TOUT, true>(pipe, out_ptr(j), in_ptr(in, me, j), w, nw, cnt, a.scale)) return;
+      if (!lane_reduce<TIN, TIN, TOUT, true, RAGGED>(pipe, out_ptr(j), in_ptr(in, me, j), w, nw, cnt, a.scale)) return;
     }
     cta_signal_mask(g, c, kSlotExit, others);
     cta_wait_mask(g, c, kSlotExit, others);
@@ -393,24 +394,24 @@ __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, 
         if (t < n) {
           char* d = stage_ptr(s.dst, rs_stage_offset(algo, P, t) + (b - s.send_first), j);
           if (nw == 0 && TW == TIN) {
-            if (!lane_copy1<false>(pipe, d, in_ptr(in, b, j), cnt * SI)) return;
-          } else {
-            cta_reduce<TIN, TW, TW, true>(&d, 1, in_ptr(in, b, j), w, nw, cnt, 1.0f);
+            if (!lane_copy1<false, RAGGED>(pipe, d, in_ptr(in, b, j), cnt * SI)) return;
+          } else if (!lane_reduce<TIN, TW, TW, true, RAGGED>(pipe, d, in_ptr(in, b, j), w, nw, cnt, 1.0f)) {
+            return;
           }
         } else {
-          if (!lane_reduce<TIN, TW, TOUT, true>(pipe, out_ptr(j), in_ptr(in, b, j), w, nw, cnt, a.scale)) return;
+          if (!lane_reduce<TIN, TW, TOUT, true, RAGGED>(pipe, out_ptr(j), in_ptr(in, b, j), w, nw, cnt, a.scale)) return;
         }
       }
-    if (t < n) publish(g, c, step_kind(algo, t), s.dst);
+    if (t < n) publish(pipe, g, c, step_kind(algo, t), s.dst);
   }
 }
 
-template <int TIN, int TW, int TOUT>
+template <int TIN, int TW, int TOUT, bool RAGGED>
 __global__ void __launch_bounds__(kCollThreads, 1) reduce_scatter_kernel(const __grid_constant__ ReduceScatterArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   BulkPipe pipe;
   bulk_pipe_init(pipe, smem, a.g.timeout_ns);
-  reduce_scatter_body<TIN, TW, TOUT>(a, pipe, kCollReduceScatter);
+  reduce_scatter_body<TIN, TW, TOUT, RAGGED>(a, pipe, kCollReduceScatter);
 }
 
 // ============================================================================ all-reduce = reduce-scatter + all-gather
@@ -422,13 +423,13 @@ __global__ void __launch_bounds__(kCollThreads, 1) reduce_scatter_kernel(const _
 // for one of phase two; a peer's block is pushed into this rank's tensor only after this rank has
 // signalled its entry into phase two, that is after it has read all of its own input.
 // Lanes keep the same element range in both phases (lane ranges are multiples of 8 elements).
-template <int DT>
+template <int DT, bool RAGGED>
 __global__ void __launch_bounds__(kCollThreads, 1) all_reduce_rsag_kernel(const __grid_constant__ AllReduceRsAgArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   BulkPipe pipe;
   bulk_pipe_init(pipe, smem, a.rs.g.timeout_ns);
-  reduce_scatter_body<DT, DT, DT>(a.rs, pipe, kCollAllReduce);
-  cta_bulk_flush();          // the block written by phase one is what phase two sends
+  reduce_scatter_body<DT, DT, DT, RAGGED>(a.rs, pipe, kCollAllReduce);
+  cta_bulk_flush(pipe);          // the block written by phase one is what phase two sends
   __syncthreads();
   all_gather_body(a.ag, pipe, 8 * Elem<DT>::size, kCollAllReduce);
 }
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(kCollThreads, 1) all_reduce_kernel(const __gri
       slice(s, &lo, &cnt);
       if (!lane_copy1<false>(pipe, buf + lo * S, data + lo * S, cnt * S)) return;
     }
-  publish_mask(g, c, kSlotEntry, others);
+  publish_mask(pipe, g, c, kSlotEntry, others);
   if (!cta_wait_mask(g, c, kSlotEntry, others)) return;
 
   uint64_t lo, cnt;
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(kCollThreads, 1) all_reduce_kernel(const __gri
       slice(s, &l2, &c2);
       if (!lane_copy1<true>(pipe, data + l2 * S, buf + l2 * S, c2 * S)) return;
     }
-  cta_bulk_flush();
+  cta_bulk_flush(pipe);
 }
 
 // ============================================================================ broadcast
@@ -555,12 +556,12 @@ __global__ void __launch_bounds__(kCollThreads, 1) broadcast_kernel(const __grid
       for (int k = 1; k < P; ++k) dsts[nd++] = g.heap[pmod(me + k, P)] + a.buf_off + lo;
       if (!lane_copy<false>(pipe, dsts, nd, src + lo, len)) return;
     }
-    publish_mask(g, c, kSlotStep0, others);
+    publish_mask(pipe, g, c, kSlotStep0, others);
   } else {
     cta_signal(g, c, kSlotEntry, a.root);
     if (!cta_wait(g, c, kSlotStep0, a.root)) return;
     if (data != nullptr && !lane_copy1<true>(pipe, data + lo, buf + lo, len)) return;
-    cta_bulk_flush();
+    cta_bulk_flush(pipe);
   }
 }
 
@@ -624,11 +625,27 @@ cudaError_t launch_all_gather(const AllGatherArgs& a, int nlanes, cudaStream_t s
   return launch(all_gather_kernel, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
 }
 
+// Whether some vector of a reduce-scatter would be misaligned: a block of the input, of the staging area or of the
+// result that does not start on a 16-byte boundary (an odd number of elements per block, or an offset tensor).  Such calls take the
+// kernel with the shifting loads.  It is a kernel of its own because the registers those loads need cost the aligned
+// loops a quarter of their speed (8 ranks, 6.3 M elements: 477 against 616 us); the aligned kernel sums such operands
+// element by element (8 ranks, 1000003 elements, direct: 1000 against 180 us).
+static bool rs_ragged(const ReduceScatterArgs& a) {
+  const uint64_t sw = (uint64_t)dtype_size(a.wire_dtype);
+  uint64_t m = a.dst_stride | a.out_sub_stride * (a.nsub > 1) | a.sub_stride * (a.nsub > 1);
+  if (a.algo == kPull || a.algo == kMultimem) m |= a.in_off;
+  else if (a.g.size > 1) m |= a.stage_off | a.stage_elems * sw;
+  for (int i = 0; i < a.g.nlocal; ++i) m |= (uint64_t)reinterpret_cast<uintptr_t>(a.in[i]) | (uint64_t)reinterpret_cast<uintptr_t>(a.out[i]);
+  return (m & 15u) != 0;
+}
+
 #define PCCL_RS_CASE(TI, TW_, TO)                                                              \
   if (a.in_dtype == TI && a.wire_dtype == TW_ && a.out_dtype == TO)                            \
-    return launch(reduce_scatter_kernel<TI, TW_, TO>, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
+    return rs_ragged(a) ? launch(reduce_scatter_kernel<TI, TW_, TO, true>, a, nlanes, kCollThreads, kBulkSmemBytes, stream) \
+                        : launch(reduce_scatter_kernel<TI, TW_, TO, false>, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
 
 cudaError_t launch_reduce_scatter(const ReduceScatterArgs& a, int nlanes, cudaStream_t stream) {
+  if (a.stage_elems < a.sub_elems) return cudaErrorInvalidValue;
   PCCL_RS_CASE(kBF16, kBF16, kBF16)
   PCCL_RS_CASE(kBF16, kBF16, kF32)
   PCCL_RS_CASE(kBF16, kF32, kBF16)
@@ -650,10 +667,11 @@ cudaError_t launch_all_reduce(const AllReduceArgs& a, int nlanes, cudaStream_t s
 }
 
 cudaError_t launch_all_reduce_rsag(const AllReduceRsAgArgs& a, int nlanes, cudaStream_t stream) {
+  if (a.rs.stage_elems < a.rs.sub_elems) return cudaErrorInvalidValue;
   const int dt = a.rs.in_dtype;
-  if (dt == kBF16) return launch_rsag(all_reduce_rsag_kernel<kBF16>, a, nlanes, stream);
-  if (dt == kF16) return launch_rsag(all_reduce_rsag_kernel<kF16>, a, nlanes, stream);
-  if (dt == kF32) return launch_rsag(all_reduce_rsag_kernel<kF32>, a, nlanes, stream);
+  if (dt == kBF16) return rs_ragged(a.rs) ? launch_rsag(all_reduce_rsag_kernel<kBF16, true>, a, nlanes, stream) : launch_rsag(all_reduce_rsag_kernel<kBF16, false>, a, nlanes, stream);
+  if (dt == kF16) return rs_ragged(a.rs) ? launch_rsag(all_reduce_rsag_kernel<kF16, true>, a, nlanes, stream) : launch_rsag(all_reduce_rsag_kernel<kF16, false>, a, nlanes, stream);
+  if (dt == kF32) return rs_ragged(a.rs) ? launch_rsag(all_reduce_rsag_kernel<kF32, true>, a, nlanes, stream) : launch_rsag(all_reduce_rsag_kernel<kF32, false>, a, nlanes, stream);
   return cudaErrorInvalidValue;
 }
 

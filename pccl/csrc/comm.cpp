@@ -304,6 +304,7 @@ void Comm::all_gather(int gid, AllGatherArgs a, int nlanes, cudaStream_t stream)
 }
 
 void Comm::reduce_scatter(int gid, ReduceScatterArgs a, int nlanes, cudaStream_t stream) {
+  if (a.stage_elems < a.sub_elems) a.stage_elems = a.sub_elems;
   if (a.algo == kMultimem && mc_heap_ == 0) throw Error("multimem reduce-scatter requested but no multicast mapping exists");
   if (a.algo == kRecursive && !is_pow2(group_size(gid))) throw Error("recursive halving needs a power-of-two group");
   {
@@ -312,7 +313,7 @@ void Comm::reduce_scatter(int gid, ReduceScatterArgs a, int nlanes, cudaStream_t
       check_extent(a.in_off, (P - 1) * a.dst_stride + (ns - 1) * a.sub_stride + a.sub_elems * (uint64_t)dtype_size(a.in_dtype),
                    "reduce-scatter symmetric input");
     } else if (P > 1) {
-      check_extent(a.stage_off, (P - 1) * ns * a.sub_elems * (uint64_t)dtype_size(a.wire_dtype), "reduce-scatter staging");
+      check_extent(a.stage_off, (P - 1) * ns * a.stage_elems * (uint64_t)dtype_size(a.wire_dtype), "reduce-scatter staging");
     }
   }
   const bool staged = a.algo != kPull && a.algo != kMultimem && in_staging(a.stage_off);
@@ -331,9 +332,10 @@ void Comm::all_reduce_rsag(int gid, AllReduceRsAgArgs a, int nlanes, cudaStream_
   if (a.rs.algo != a.ag.algo || (a.rs.algo != kRing && a.rs.algo != kRecursive))
     throw Error("the two-phase all-reduce runs the ring or the recursive schedules");
   if (a.rs.algo == kRecursive && !is_pow2(group_size(gid))) throw Error("recursive halving/doubling needs a power-of-two group");
+  if (a.rs.stage_elems < a.rs.sub_elems) a.rs.stage_elems = a.rs.sub_elems;
   {
     const uint64_t P = (uint64_t)group_size(gid);
-    check_extent(a.rs.stage_off, (P - 1) * a.rs.sub_elems * (uint64_t)dtype_size(a.rs.wire_dtype), "all-reduce staging of partial sums");
+    check_extent(a.rs.stage_off, (P - 1) * a.rs.stage_elems * (uint64_t)dtype_size(a.rs.wire_dtype), "all-reduce staging of partial sums");
     check_extent(a.ag.recv_off, (P - 1) * a.ag.src_stride + a.ag.sub_bytes, "all-reduce gather landing zone");
   }
   const bool staged = in_staging(a.rs.stage_off) || in_staging(a.ag.recv_off);

@@ -133,6 +133,8 @@ struct ReduceScatterArgs {
   uint64_t dst_stride;
   uint64_t sub_stride;
   uint64_t sub_elems;           // elements of one sub-block handled by this launch
+  uint64_t stage_elems;         // elements from one staged sub-block to the next: sub_elems, or that
+                                // rounded up so that every staged block starts on a 16-byte boundary
   uint64_t out_sub_stride;      // bytes between consecutive sub-blocks of `out`
   int nsub;
   float scale;

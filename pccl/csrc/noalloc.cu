@@ -105,6 +105,7 @@ extern "C" int pccl_reduce_scatter_noalloc(const void* const* inputs, void* cons
   a.dst_stride = block_elems * (uint64_t)dtype_size(in_dtype);
   a.sub_stride = 0;
   a.sub_elems = block_elems;
+  a.stage_elems = block_elems;
   a.out_sub_stride = block_elems * (uint64_t)dtype_size(out_dtype);
   a.nsub = 1;
   a.scale = scale;

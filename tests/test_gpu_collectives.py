@@ -122,6 +122,67 @@ def test_reduce_scatter_pull_symmetric_input(P):
     del sym
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n", [1, 249, 4099, 31 * 16 * 8 * 3 + 13])
+@pytest.mark.parametrize("shift", [0, 3])
+def test_misaligned_blocks(dtype, n, shift):
+    """Blocks that start anywhere within 16 bytes (odd counts, tensors behind an offset): the shifting loads of the
+    all-gather, reduce-scatter and all-reduce, at the ends of vectors, of warps and of block passes, for private
+    and symmetric buffers; nothing next to the results may change."""
+    P = 4
+    comm = emu(P)
+    gid = comm.world_group.gid
+
+    def framed(count, dt, fill=None):
+        store = torch.full((count + shift + 16,), 7.0, dtype=dt, device=DEV)
+        view = store[shift:shift + count]
+        if fill is not None:
+            view.copy_(fill)
+        return store, view
+
+    def intact(stores, count):
+        return all(bool((s[:shift] == 7.0).all()) and bool((s[shift + count:] == 7.0).all()) for s in stores)
+
+    vals = [rand(n, dtype, 900 + r) for r in range(P)]
+    want = torch.cat(vals)
+    for algo in (sch.DIRECT, sch.RING, sch.PULL):
+        ins = [framed(n, dtype, v)[1] for v in vals]
+        stores, outs = zip(*[framed(P * n, dtype) for _ in range(P)])
+        comm.native.all_gather(gid, list(outs), ins, sch.ALGO_IDS[algo], 3)
+        comm.check()
+        assert all(torch.equal(o, want) for o in outs) and intact(stores, P * n), algo
+    sym = comm.empty(P * n, dtype)
+    comm.native.all_gather(gid, sym, vals, sch.ALGO_IDS[sch.RECURSIVE], 3)
+    comm.check()
+    assert all(torch.equal(o, want) for o in sym)
+
+    full = [rand(P * n, dtype, 950 + r) for r in range(P)]
+    for r in range(P):
+        sym[r].copy_(full[r])
+    ref = [t for t in (sum(t.double() for t in full) / P).view(P, n)]
+    for algo in (sch.DIRECT, sch.RING, sch.RECURSIVE, sch.PULL):
+        ins = sym if algo == sch.PULL else [framed(P * n, dtype, v)[1] for v in full]
+        stores, outs = zip(*[framed(n, torch.float32) for _ in range(P)])
+        comm.native.reduce_scatter(gid, list(outs), ins, sch.ALGO_IDS[algo], 3, 1.0 / P, None)
+        comm.check()
+        # the direct and pull forms sum in fp32 and round nothing to 16 bits; a ring or a halving rounds its partial sums
+        tol = 1e-5 if dtype == torch.float32 or algo in (sch.DIRECT, sch.PULL) else 3e-2
+        for r in range(P):
+            torch.testing.assert_close(outs[r].double(), ref[r], rtol=tol, atol=tol)
+        assert intact(stores, n), algo
+    same = [rand(P * n, dtype, 970 + r) for r in range(P)]
+    mean = sum(t.double() for t in same) / P
+    for algo in (sch.DIRECT, sch.RING, sch.RECURSIVE):
+        stores, ts = zip(*[framed(P * n, dtype, v) for v in same])
+        comm.native.all_reduce(gid, list(ts), sch.ALGO_IDS[algo], 3, 1.0 / P)
+        comm.check()
+        tol = 1e-5 if dtype == torch.float32 else 3e-2
+        for r in range(P):
+            torch.testing.assert_close(ts[r].double(), mean, rtol=tol, atol=tol)
+        assert intact(stores, P * n), algo
+    del sym
+
+
 def test_reduce_scatter_bf16_accumulates_in_fp32():
     """Many equal small addends: a 16-bit accumulator would stall, fp32 does not."""
     P = 8
