@@ -1000,8 +1000,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
       }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * BN;
+      bool ready = false;                       // the stage was seen full behind the last k-block's MMAs
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!gemm_wait(full + st, ph, abort_flag)) {
+        if (!ready && !gemm_wait(full + st, ph, abort_flag)) {
           ok = false;
           break;
         }
@@ -1014,11 +1015,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
           for (int k = 0; k < BK / 16; ++k)
             mma_bf16_pair(d_tmem + BN, da + (kHalfBytes >> 4) + k * a_step, db + k * b_step, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
         }
-        mma_commit_pair(empty0 + st * 8);       // free the stage in both CTAs
+        const uint32_t freed = empty0 + st * 8;
         if (++st == (uint32_t)NST) {
           st = 0;
           ph ^= 1u;
         }
+        ready = kb + 1 < kb1 && mbar_try_wait(full + st, ph);
+        mma_commit_pair(freed);                 // free the stage in both CTAs
       }
       if (!ok) break;
       mma_commit_pair(smem_u32(tmem_full + acc));      // accumulator complete: wake both epilogues
