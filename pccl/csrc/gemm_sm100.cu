@@ -703,15 +703,11 @@ __device__ __forceinline__ int sk_pair_of(int i, int I, int G) { return (int)((u
 // to bf16 and writes them to the warp's piece of shared memory in the 128-byte-swizzled layout (16-byte
 // chunk c of row l at chunk c ^ (l % 8)).  bias_s: this slab's 64 bias values in shared memory, or nullptr.
 // KEEP: the packed pairs stay in r[0..32) for a second output.
-// Both halves of a pair of fp32 values in one instruction.
-__device__ __forceinline__ void add_pair(uint32_t& x, uint32_t& y, uint32_t bx, uint32_t by) {
-  asm("{\n\t.reg .b64 p, q;\n\t"
-      "mov.b64 p, {%0, %1};\n\t"
-      "mov.b64 q, {%2, %3};\n\t"
-      "add.rn.f32x2 p, p, q;\n\t"
-      "mov.b64 {%0, %1}, p;\n\t}"
-      : "+r"(x), "+r"(y)
-      : "r"(bx), "r"(by));
+__device__ __forceinline__ void add_pair(uint32_t& x, uint32_t& y, uint32_t bias_pair) {
+  float a, b;
+  split(f2(__uint_as_float(x), __uint_as_float(y)) + unpack2(bias_pair), a, b);
+  x = __float_as_uint(a);
+  y = __float_as_uint(b);
 }
 template <bool BIAS, bool KEEP>
 __device__ __forceinline__ void slab_to_smem(uint32_t (&r)[64], unsigned char* buf, const unsigned char* bias_s, int lane) {
@@ -723,7 +719,7 @@ __device__ __forceinline__ void slab_to_smem(uint32_t (&r)[64], unsigned char* b
       const uint4 q = *reinterpret_cast<const uint4*>(bias_s + c * 16);
       const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) add_pair(r[c * 8 + 2 * e], r[c * 8 + 2 * e + 1], qw[e] << 16, qw[e] & 0xffff0000u);
+      for (int e = 0; e < 4; ++e) add_pair(r[c * 8 + 2 * e], r[c * 8 + 2 * e + 1], qw[e]);
     }
     uint32_t w[4];
 #pragma unroll
@@ -744,8 +740,9 @@ __device__ __forceinline__ void slab_gelu_to_smem(const uint32_t (&r)[64], unsig
     uint32_t w[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const uint32_t v = r[c * 4 + e];
-      const __nv_bfloat162 h = __floats2bfloat162_rn(gelu_tanh(__uint_as_float(v << 16)), gelu_tanh(__uint_as_float(v & 0xffff0000u)));
+      float g0, g1;
+      split(gelu_tanh2(unpack2(r[c * 4 + e])), g0, g1);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(g0, g1);
       w[e] = *reinterpret_cast<const uint32_t*>(&h);
     }
     *reinterpret_cast<uint4*>(row + (((uint32_t)c ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -1334,7 +1331,9 @@ __device__ __forceinline__ void tile_reduce_store(const TileArgs& a, uint32_t ti
       const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
       w[e] = *reinterpret_cast<const uint32_t*>(&h);
       if (a.act_out != nullptr) {
-        const __nv_bfloat162 hg = __floats2bfloat162_rn(gelu_tanh(__low2float(h)), gelu_tanh(__high2float(h)));
+        float g0, g1;
+        split(gelu_tanh2(unpack2(w[e])), g0, g1);
+        const __nv_bfloat162 hg = __floats2bfloat162_rn(g0, g1);
         g[e] = *reinterpret_cast<const uint32_t*>(&hg);
       }
     }

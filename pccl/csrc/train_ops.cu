@@ -37,53 +37,63 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 __device__ __forceinline__ float round_bf16(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
 
 // ---------------------------------------------------------------- column sum
-// out[c] = sum_r X[r, c]; X is [T, N] bf16 row-major with N % 8 == 0.  A block covers 512
-// columns (64 threads x 16 bytes: 1 KiB of one row, so a warp reads 512 contiguous bytes) in
-// four row lanes, and one slice of the rows; the last block to finish a column tile adds the
-// slices' fp32 partial sums and writes bf16.
+// out[c] = sum_r X[r, c]; X is [T, N] bf16 row-major with N % 8 == 0.  A block covers 256
+// columns (a warp reads 512 contiguous bytes of one row) in eight row lanes, one per warp, and one slice of the
+// rows; the last block to finish a column tile adds the slices' fp32 partial sums and writes bf16.  That
+// last sum is a chain of loads from one SM at the end of everything, so the slices are few (col_sum_row_splits) and
+// each thread keeps four of them in flight (more would cost the main loop its fourth block per SM).  Measured against 512-column tiles and up to 296 slices: 4096 x 1024
+// 18.8 -> 5.6 us; GELU form 4096 x 4096 26.4 -> 20.4 us, with its arithmetic in pairs of elements.
 // GELU form: X is the gradient of the GELU's output and U its input; the kernel writes
 // DU = X * gelu'(U) and sums the columns of DU (as rounded to bf16), the bias gradient of
 // the linear layer in front of the GELU.
 // Concatenating form: the columns are those of three [T, N/3] matrices side by side (the
 // gradients of q, k and v); the kernel writes the [T, N] concatenation to DU while it sums.
-constexpr int kColTile = 512, kRowLanes = 4;
+constexpr int kColTile = 256, kRowLanes = 8;
 enum ColMode { kColSum = 0, kColGelu = 1, kColCat3 = 2 };
 
 template <int MODE>
-__device__ __forceinline__ void col_item(const uint4& q, const uint4& uq, __nv_bfloat16* DU, int64_t off, float* acc) {
-  float f[8];
-  unpack8(q, f);
+__device__ __forceinline__ void col_item(const uint4& q, const uint4& uq, __nv_bfloat16* DU, int64_t off, F2 (&acc)[4]) {
   if (MODE == kColGelu) {
-    float u[8];
-    unpack8(uq, u);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w}, uw[4] = {uq.x, uq.y, uq.z, uq.w};
+    uint32_t o[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] *= gelu_tanh_grad(u[e]);
-    const uint4 packed = pack8(f);               // one rounding; the sums below are of the rounded values
-    *reinterpret_cast<uint4*>(DU + off) = packed;
-    unpack8(packed, f);
+    for (int e = 0; e < 4; ++e) {
+      // the clamp of gelu_tanh_grad, on the packed pair (as there, NaN goes to a bound)
+      __nv_bfloat162 u = *reinterpret_cast<const __nv_bfloat162*>(&uw[e]);
+      u = __hmin2(__hmax2(u, __float2bfloat162_rn(-20.f)), __float2bfloat162_rn(20.f));
+      float a, b;
+      split(unpack2(w[e]) * gelu_tanh_grad2(unpack2(*reinterpret_cast<const uint32_t*>(&u))), a, b);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);     // one rounding; the sums are of the rounded values
+      o[e] = *reinterpret_cast<const uint32_t*>(&h);
+      acc[e] = acc[e] + unpack2(o[e]);
+    }
+    *reinterpret_cast<uint4*>(DU + off) = make_uint4(o[0], o[1], o[2], o[3]);
+    return;
   }
   if (MODE == kColCat3) *reinterpret_cast<uint4*>(DU + off) = q;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] += f[e];
+  acc[0] = acc[0] + unpack2(q.x);
+  acc[1] = acc[1] + unpack2(q.y);
+  acc[2] = acc[2] + unpack2(q.z);
+  acc[3] = acc[3] + unpack2(q.w);
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256) col_sum_kernel(const __nv_bfloat16* __restrict__ X, int64_t T, int N,
+__global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* __restrict__ X, int64_t T, int N,
                                                       __nv_bfloat16* __restrict__ out, float* __restrict__ partial,
                                                       int* __restrict__ counters, const __nv_bfloat16* __restrict__ U,
                                                       __nv_bfloat16* __restrict__ DU, const __nv_bfloat16* __restrict__ X2) {
   __shared__ __align__(16) float red[kRowLanes][kColTile];
   __shared__ int s_last;
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col_base = blockIdx.x * kColTile;
   const int col = col_base + tx * 8;
   const int R = gridDim.y;
   const int64_t rows_per = (T + R - 1) / R;
   const int64_t r0 = (int64_t)blockIdx.y * rows_per;
   const int64_t r1 = r0 + rows_per < T ? r0 + rows_per : T;
-  float acc[8];
+  F2 acc[4];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+  for (int e = 0; e < 4; ++e) acc[e] = f2(0.f);
   if (col < N) {
     // where this thread's 8 columns come from: X itself, or one of the three sources
     const __nv_bfloat16* src = X + col;
@@ -110,49 +120,52 @@ __global__ void __launch_bounds__(256) col_sum_kernel(const __nv_bfloat16* __res
       col_item<MODE>(q, uq, DU, r * N + col, acc);
     }
   }
-  *reinterpret_cast<float4*>(&red[ty][tx * 8]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-  *reinterpret_cast<float4*>(&red[ty][tx * 8 + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-  __syncthreads();
-  for (int c = threadIdx.x; c < kColTile; c += 256)
-    if (col_base + c < N) partial[(int64_t)blockIdx.y * N + col_base + c] = red[0][c] + red[1][c] + red[2][c] + red[3][c];
+  // the eight row lanes' sums, column by column (256 threads, 256 columns)
+  auto combine = [&]() {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split(acc[e], red[ty][tx * 8 + 2 * e], red[ty][tx * 8 + 2 * e + 1]);
+    __syncthreads();
+    float a = red[0][threadIdx.x];
+#pragma unroll
+    for (int l = 1; l < kRowLanes; ++l) a += red[l][threadIdx.x];
+    return a;
+  };
+  const int mine = col_base + threadIdx.x;
+  const float part = combine();
+  if (mine < N) __stcg(partial + (int64_t)blockIdx.y * N + mine, part);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_last = atomicAdd(counters + blockIdx.x, 1) == R - 1;
   __syncthreads();
   if (s_last) {
     __threadfence();
-    // the four row lanes split the slices; every thread adds 8 columns of its share
+    // the row lanes split the slices; every thread adds 8 columns of its share, four slices at a time
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    for (int e = 0; e < 4; ++e) acc[e] = f2(0.f);
     if (col < N) {
-      int y = ty;
-      for (; y + 3 * kRowLanes < R; y += 4 * kRowLanes) {
+      for (int y0 = ty; y0 < R; y0 += 4 * kRowLanes) {
         float4 v[8];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const float* src = partial + (int64_t)(y + k * kRowLanes) * N + col;
-          v[2 * k] = __ldcg(reinterpret_cast<const float4*>(src));
-          v[2 * k + 1] = __ldcg(reinterpret_cast<const float4*>(src + 4));
+          const int y = y0 + k * kRowLanes;
+          const float* src = partial + (int64_t)y * N + col;
+          v[2 * k] = v[2 * k + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (y < R) {
+            v[2 * k] = __ldcg(reinterpret_cast<const float4*>(src));
+            v[2 * k + 1] = __ldcg(reinterpret_cast<const float4*>(src + 4));
+          }
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          acc[0] += v[2 * k].x, acc[1] += v[2 * k].y, acc[2] += v[2 * k].z, acc[3] += v[2 * k].w;
-          acc[4] += v[2 * k + 1].x, acc[5] += v[2 * k + 1].y, acc[6] += v[2 * k + 1].z, acc[7] += v[2 * k + 1].w;
+          acc[0] = acc[0] + f2(v[2 * k].x, v[2 * k].y);
+          acc[1] = acc[1] + f2(v[2 * k].z, v[2 * k].w);
+          acc[2] = acc[2] + f2(v[2 * k + 1].x, v[2 * k + 1].y);
+          acc[3] = acc[3] + f2(v[2 * k + 1].z, v[2 * k + 1].w);
         }
       }
-      for (; y < R; y += kRowLanes) {
-        const float* src = partial + (int64_t)y * N + col;
-        const float4 v0 = __ldcg(reinterpret_cast<const float4*>(src)), v1 = __ldcg(reinterpret_cast<const float4*>(src + 4));
-        acc[0] += v0.x, acc[1] += v0.y, acc[2] += v0.z, acc[3] += v0.w;
-        acc[4] += v1.x, acc[5] += v1.y, acc[6] += v1.z, acc[7] += v1.w;
-      }
     }
-    __syncthreads();
-    *reinterpret_cast<float4*>(&red[ty][tx * 8]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    *reinterpret_cast<float4*>(&red[ty][tx * 8 + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-    __syncthreads();
-    for (int c = threadIdx.x; c < kColTile; c += 256)
-      if (col_base + c < N) out[col_base + c] = __float2bfloat16_rn(red[0][c] + red[1][c] + red[2][c] + red[3][c]);
+    const float total = combine();
+    if (mine < N) out[mine] = __float2bfloat16_rn(total);
     if (threadIdx.x == 0) counters[blockIdx.x] = 0;   // ready for the next call
   }
 }
@@ -450,6 +463,18 @@ __global__ void __launch_bounds__(256) ln_bwd_finalize_kernel(LnBwdFinalizeArgs 
 }
 
 // ---------------------------------------------------------------- GELU forward
+__device__ __forceinline__ uint4 gelu8(const uint4& q) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float a, b;
+    split(gelu_tanh2(unpack2(w[e])), a, b);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    o[e] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int64_t nvec) {
   const int64_t stride = (int64_t)gridDim.x * 256;
   int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -458,21 +483,9 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__
 #pragma unroll
     for (int k = 0; k < 4; ++k) q[k] = in[i + k * stride];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float f[8];
-      unpack8(q[k], f);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = gelu_tanh(f[e]);
-      out[i + k * stride] = pack8(f);
-    }
+    for (int k = 0; k < 4; ++k) out[i + k * stride] = gelu8(q[k]);
   }
-  for (; i < nvec; i += stride) {
-    float f[8];
-    unpack8(in[i], f);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = gelu_tanh(f[e]);
-    out[i] = pack8(f);
-  }
+  for (; i < nvec; i += stride) out[i] = gelu8(in[i]);
 }
 
 // ---------------------------------------------------------------- residual add + layer norm
@@ -546,8 +559,9 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const __nv_bfloat16* __rest
 
 int col_sum_row_splits(int64_t T, int N) {
   const int tiles = (N + kColTile - 1) / kColTile;
-  int R = (148 * 4 + tiles - 1) / tiles;                       // about four blocks per SM (3, 5 and 6 measured slower)
-  const int64_t max_r = (T + 4 * kRowLanes - 1) / (4 * kRowLanes);
+  int R = 148 * 4 / tiles;                                     // four blocks per SM and no second wave
+  if (R > 8 * kRowLanes) R = 8 * kRowLanes;                    // the last sum in two rounds of loads
+  const int64_t max_r = (T + 2 * kRowLanes - 1) / (2 * kRowLanes);
   if (R > max_r) R = (int)max_r;
   if (R < 1) R = 1;
   return R;
