@@ -25,6 +25,7 @@
 #include "bulk.cuh"
 #include "act.cuh"
 #include "gemm.h"
+#include "pdl.cuh"
 #include "primitives.cuh"
 
 namespace pccl {
@@ -870,6 +871,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
 
   cluster_wait();                           // both CTAs' barriers exist before anyone signals across
   tc_fence_after();
+  pdl_wait();                               // operands complete, outputs no longer read: every role may start its (bounded) waits
+  if (!fused) pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
@@ -1384,6 +1387,7 @@ __global__ void __launch_bounds__(kTileThreads, TileCfg<TN>::kPerSm)
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
+    pdl_wait();
     for (int i = 0; i < n && i < Cfg::kStages; ++i) load(i, i);      // the barriers they signal are this thread's own
   } else if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)TN)
@@ -1393,6 +1397,8 @@ __global__ void __launch_bounds__(kTileThreads, TileCfg<TN>::kPerSm)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
@@ -1556,8 +1562,9 @@ cudaError_t launch_pair(const CUtensorMap& mA, const CUtensorMap& mW, const CUte
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  gemm_sm100_2cta_kernel<A_MN, B_MN, WIDE><<<grid, kGemm2Threads, kGemm2Smem, stream>>>(mA, mW, mOwn, mC, mAct, a);
-  return cudaGetLastError();
+  // a fused launch waits for panels that peers or copy engines bring: nothing may take its place on the device early
+  return launch_pdl(gemm_sm100_2cta_kernel<A_MN, B_MN, WIDE>, grid, kGemm2Threads, kGemm2Smem, stream, 0u, a.panel_flags == nullptr, mA, mW,
+                    mOwn, mC, mAct, a);
 }
 
 template <bool A_MN, bool B_MN, int TN>
@@ -1571,19 +1578,8 @@ cudaError_t launch_tile_form(const CUtensorMap& mA, const CUtensorMap& mW, const
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * ta.split));
-  cfg.blockDim = dim3(kTileThreads);
-  cfg.dynamicSmemBytes = TileCfg<TN>::kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)ta.split;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, gemm_sm100_tile_kernel<A_MN, B_MN, TN>, mA, mW, ta);
-  return e != cudaSuccess ? e : cudaGetLastError();
+  return launch_pdl(gemm_sm100_tile_kernel<A_MN, B_MN, TN>, tiles * ta.split, kTileThreads, TileCfg<TN>::kSmem, stream,
+                    (unsigned)ta.split, true, mA, mW, ta);
 }
 
 template <int TN>

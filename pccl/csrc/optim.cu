@@ -13,6 +13,7 @@
 
 #include "act.cuh"
 #include "optim.h"
+#include "pdl.cuh"
 
 namespace pccl {
 
@@ -68,6 +69,8 @@ __device__ __forceinline__ float sq8<float>(const uint4& q) {
 template <typename T>
 __global__ void __launch_bounds__(kOptThreads) sq_norm_kernel(const T* __restrict__ x, uint64_t n, float* out) {
   __shared__ float red[32];
+  pdl_wait();
+  pdl_trigger();
   constexpr uint64_t EPV = 16 / sizeof(T);
   float acc = 0.f;
   uint64_t done = 0;
@@ -100,6 +103,8 @@ template <typename G>
 __global__ void __launch_bounds__(kOptThreads)
     adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v, const G* __restrict__ grad,
                  __nv_bfloat16* __restrict__ param, uint64_t n, AdamWArgs a, const float* total_sq_norm) {
+  pdl_wait();
+  pdl_trigger();
   float clip = 1.0f;
   if (total_sq_norm != nullptr && a.max_grad_norm > 0.f) {
     const float norm = sqrtf(*total_sq_norm) * a.grad_scale;
@@ -197,6 +202,8 @@ template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
                                                             float* loss_sum, int64_t rows, int vocab, int64_t row_stride,
                                                             float grad_scale, int64_t ignore_index, int* bad_targets) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* row_s = reinterpret_cast<uint4*>(smem_raw);
   __nv_bfloat16* tail_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);
@@ -366,9 +373,8 @@ int grid_for(uint64_t n, int threads, int per_thread) {
 cudaError_t launch_sq_norm(const void* x, int dtype_is_bf16, uint64_t n, float* out, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const int grid = grid_for(n, kOptThreads, 16);
-  if (dtype_is_bf16) sq_norm_kernel<<<grid, kOptThreads, 0, s>>>((const __nv_bfloat16*)x, n, out);
-  else sq_norm_kernel<<<grid, kOptThreads, 0, s>>>((const float*)x, n, out);
-  return cudaGetLastError();
+  if (dtype_is_bf16) return launch_pdl(sq_norm_kernel<__nv_bfloat16>, grid, kOptThreads, 0, s, (const __nv_bfloat16*)x, n, out);
+  return launch_pdl(sq_norm_kernel<float>, grid, kOptThreads, 0, s, (const float*)x, n, out);
 }
 
 cudaError_t launch_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf16, void* param_bf16,
@@ -376,12 +382,10 @@ cudaError_t launch_adamw(float* master, float* m, float* v, const void* grad, in
   if (n == 0) return cudaSuccess;
   const int grid = grid_for(n, kOptThreads, 8);
   if (grad_is_bf16)
-    adamw_kernel<<<grid, kOptThreads, 0, s>>>(master, m, v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)param_bf16, n, a,
-                                              total_sq_norm);
-  else
-    adamw_kernel<<<grid, kOptThreads, 0, s>>>(master, m, v, (const float*)grad, (__nv_bfloat16*)param_bf16, n, a,
-                                              total_sq_norm);
-  return cudaGetLastError();
+    return launch_pdl(adamw_kernel<__nv_bfloat16>, grid, kOptThreads, 0, s, master, m, v, (const __nv_bfloat16*)grad,
+                      (__nv_bfloat16*)param_bf16, n, a, total_sq_norm);
+  return launch_pdl(adamw_kernel<float>, grid, kOptThreads, 0, s, master, m, v, (const float*)grad, (__nv_bfloat16*)param_bf16, n,
+                    a, total_sq_norm);
 }
 
 cudaError_t launch_ce_fwd_bwd(void* logits_bf16, const int64_t* targets, float* loss_sum, int64_t rows, int vocab,
@@ -405,13 +409,9 @@ cudaError_t launch_ce_fwd_bwd(void* logits_bf16, const int64_t* targets, float* 
   const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(1024 / threads, (int64_t)(228 * 1024 / (smem + 1280))));
   const unsigned grid = (unsigned)std::min<int64_t>(rows, 148 * per_sm);
   auto* l = (__nv_bfloat16*)logits_bf16;
-  if (threads == 512)
-    ce_fwd_bwd_kernel<512><<<grid, 512, smem, s>>>(l, targets, loss_sum, rows, vocab, row_stride, grad_scale, ignore_index, bad_targets);
-  else if (threads == 256)
-    ce_fwd_bwd_kernel<256><<<grid, 256, smem, s>>>(l, targets, loss_sum, rows, vocab, row_stride, grad_scale, ignore_index, bad_targets);
-  else
-    ce_fwd_bwd_kernel<128><<<grid, 128, smem, s>>>(l, targets, loss_sum, rows, vocab, row_stride, grad_scale, ignore_index, bad_targets);
-  return cudaGetLastError();
+  if (threads == 512) return launch_pdl(ce_fwd_bwd_kernel<512>, grid, 512, smem, s, l, targets, loss_sum, rows, vocab, row_stride, grad_scale, ignore_index, bad_targets);
+  if (threads == 256) return launch_pdl(ce_fwd_bwd_kernel<256>, grid, 256, smem, s, l, targets, loss_sum, rows, vocab, row_stride, grad_scale, ignore_index, bad_targets);
+  return launch_pdl(ce_fwd_bwd_kernel<128>, grid, 128, smem, s, l, targets, loss_sum, rows, vocab, row_stride, grad_scale, ignore_index, bad_targets);
 }
 
 }  // namespace pccl

@@ -11,6 +11,7 @@
 
 #include "act.cuh"
 #include "optim.h"
+#include "pdl.cuh"
 
 namespace pccl {
 
@@ -84,6 +85,8 @@ __global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* __
                                                       __nv_bfloat16* __restrict__ DU, const __nv_bfloat16* __restrict__ X2) {
   __shared__ __align__(16) float red[kRowLanes][kColTile];
   __shared__ int s_last;
+  pdl_wait();
+  pdl_trigger();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col_base = blockIdx.x * kColTile;
   const int col = col_base + tx * 8;
@@ -217,6 +220,8 @@ __global__ void __launch_bounds__(256, 1)
   constexpr int NV = EPT / 8;
   __shared__ float red[2][RB][4][2];
   __shared__ __align__(16) float comb[128 * EPT];
+  pdl_wait();
+  pdl_trigger();
   const int rg = threadIdx.x >> 7, t = threadIdx.x & 127, warp_in_rg = t >> 5, lane = t & 31;
   uint4 pgam[NV];
   float dgam[EPT], dbet[EPT], dxs[EPT];
@@ -333,6 +338,8 @@ __global__ void __launch_bounds__(256, 2)
                          const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ resid,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ pgamma, float* __restrict__ pbeta,
                          float* __restrict__ pdx, int64_t T) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int d = 2048;
   __shared__ float red[RB][8][2];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -438,6 +445,8 @@ struct LnBwdFinalizeArgs {
 
 __global__ void __launch_bounds__(256) ln_bwd_finalize_kernel(LnBwdFinalizeArgs f, int nparts, int d) {
   __shared__ float sa[8][33];
+  pdl_wait();
+  pdl_trigger();
   const float* __restrict__ part = f.part[blockIdx.y];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -476,6 +485,8 @@ __device__ __forceinline__ uint4 gelu8(const uint4& q) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int64_t nvec) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t stride = (int64_t)gridDim.x * 256;
   int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   for (; i + 3 * stride < nvec; i += 4 * stride) {
@@ -511,6 +522,8 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const __nv_bfloat16* __rest
                                                      float eps) {
   constexpr int NV = EPT / 8;
   __shared__ float red[4];
+  pdl_wait();
+  pdl_trigger();
   const int t = threadIdx.x;
   const float inv_d = 1.0f / (float)d;
   for (int64_t r = blockIdx.x; r < T; r += gridDim.x) {
@@ -572,9 +585,8 @@ cudaError_t launch_col_sum(const void* X, int64_t T, int N, void* out, float* pa
   if (T <= 0 || N <= 0) return cudaSuccess;
   if (N % 8 != 0) return cudaErrorInvalidValue;
   dim3 grid((N + kColTile - 1) / kColTile, R);
-  col_sum_kernel<kColSum><<<grid, 256, 0, s>>>((const __nv_bfloat16*)X, T, N, (__nv_bfloat16*)out, partial, counters, nullptr,
+  return launch_pdl(col_sum_kernel<kColSum>, grid, 256, 0, s, (const __nv_bfloat16*)X, T, N, (__nv_bfloat16*)out, partial, counters, nullptr,
                                                nullptr, nullptr);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_gelu_bwd_col_sum(const void* dg, const void* u, void* du, int64_t T, int N, void* out, float* partial,
@@ -582,9 +594,8 @@ cudaError_t launch_gelu_bwd_col_sum(const void* dg, const void* u, void* du, int
   if (T <= 0 || N <= 0) return cudaSuccess;
   if (N % 8 != 0) return cudaErrorInvalidValue;
   dim3 grid((N + kColTile - 1) / kColTile, R);
-  col_sum_kernel<kColGelu><<<grid, 256, 0, s>>>((const __nv_bfloat16*)dg, T, N, (__nv_bfloat16*)out, partial, counters,
+  return launch_pdl(col_sum_kernel<kColGelu>, grid, 256, 0, s, (const __nv_bfloat16*)dg, T, N, (__nv_bfloat16*)out, partial, counters,
                                                 (const __nv_bfloat16*)u, (__nv_bfloat16*)du, nullptr);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_cat3_col_sum(const void* a, const void* b, const void* c, void* cat, int64_t T, int N, void* out,
@@ -592,9 +603,8 @@ cudaError_t launch_cat3_col_sum(const void* a, const void* b, const void* c, voi
   if (T <= 0 || N <= 0) return cudaSuccess;
   if (N % 24 != 0) return cudaErrorInvalidValue;          // three sources of a multiple of 8 columns each
   dim3 grid((N + kColTile - 1) / kColTile, R);
-  col_sum_kernel<kColCat3><<<grid, 256, 0, s>>>((const __nv_bfloat16*)a, T, N, (__nv_bfloat16*)out, partial, counters,
+  return launch_pdl(col_sum_kernel<kColCat3>, grid, 256, 0, s, (const __nv_bfloat16*)a, T, N, (__nv_bfloat16*)out, partial, counters,
                                                 (const __nv_bfloat16*)b, (__nv_bfloat16*)cat, (const __nv_bfloat16*)c);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_gelu_fwd(const void* in, void* out, int64_t n, cudaStream_t s) {
@@ -603,8 +613,7 @@ cudaError_t launch_gelu_fwd(const void* in, void* out, int64_t n, cudaStream_t s
   const int64_t nvec = n / 8;
   int64_t blocks = (nvec + 256 * 4 - 1) / (256 * 4);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  gelu_fwd_kernel<<<(int)blocks, 256, 0, s>>>((const uint4*)in, (uint4*)out, nvec);
-  return cudaGetLastError();
+  return launch_pdl(gelu_fwd_kernel, (int)blocks, 256, 0, s, (const uint4*)in, (uint4*)out, nvec);
 }
 
 cudaError_t launch_ln_fwd(const void* x, void* branch, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
@@ -616,13 +625,14 @@ cudaError_t launch_ln_fwd(const void* x, void* branch, const void* gamma, const 
   auto* G = (const __nv_bfloat16*)gamma;
   auto* Be = (const __nv_bfloat16*)beta;
   auto* Y = (__nv_bfloat16*)y;
+  cudaError_t e = cudaSuccess;
   switch (d / 128) {
-    case 8: ln_fwd_kernel<8><<<(int)blocks, 128, 0, s>>>(X, B, G, Be, Y, mean, rstd, T, d, eps); break;
-    case 16: ln_fwd_kernel<16><<<(int)blocks, 128, 0, s>>>(X, B, G, Be, Y, mean, rstd, T, d, eps); break;
-    case 32: ln_fwd_kernel<32><<<(int)blocks, 128, 0, s>>>(X, B, G, Be, Y, mean, rstd, T, d, eps); break;
+    case 8: e = launch_pdl(ln_fwd_kernel<8>, (int)blocks, 128, 0, s, X, B, G, Be, Y, mean, rstd, T, d, eps); break;
+    case 16: e = launch_pdl(ln_fwd_kernel<16>, (int)blocks, 128, 0, s, X, B, G, Be, Y, mean, rstd, T, d, eps); break;
+    case 32: e = launch_pdl(ln_fwd_kernel<32>, (int)blocks, 128, 0, s, X, B, G, Be, Y, mean, rstd, T, d, eps); break;
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+  return e;
 }
 
 int ln_bwd_blocks() { return 296; }      // at most two blocks per SM; each leaves one partial row per array
@@ -645,19 +655,18 @@ cudaError_t launch_ln_bwd(const void* dy, const void* x, const float* mean, cons
   float* pgamma = scratch;
   float* pbeta = scratch + (int64_t)ln_bwd_blocks() * d;
   float* pdx = dx_col_sum != nullptr ? scratch + 2 * (int64_t)ln_bwd_blocks() * d : nullptr;
+  cudaError_t e = cudaSuccess;
   switch (d / 128) {
-    case 8: ln_bwd_kernel<8, 4><<<blocks, 256, 0, s>>>(DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T, d); break;
-    case 16: ln_bwd_row256_kernel<4><<<blocks, 256, 0, s>>>(DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
-    case 32: ln_bwd_kernel<32, 1><<<blocks, 256, 0, s>>>(DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T, d); break;
+    case 8: e = launch_pdl(ln_bwd_kernel<8, 4>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T, d); break;
+    case 16: e = launch_pdl(ln_bwd_row256_kernel<4>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
+    case 32: e = launch_pdl(ln_bwd_kernel<32, 1>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T, d); break;
     default: return cudaErrorInvalidValue;
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   LnBwdFinalizeArgs f;
   f.part[0] = pgamma, f.part[1] = pbeta, f.part[2] = pdx;
   f.out[0] = (__nv_bfloat16*)dgamma, f.out[1] = (__nv_bfloat16*)dbeta, f.out[2] = (__nv_bfloat16*)dx_col_sum;
-  ln_bwd_finalize_kernel<<<dim3((d + 31) / 32, pdx != nullptr ? 3 : 2), 256, 0, s>>>(f, blocks, d);
-  return cudaGetLastError();
+  return launch_pdl(ln_bwd_finalize_kernel, dim3((d + 31) / 32, pdx != nullptr ? 3 : 2), 256, 0, s, f, blocks, d);
 }
 
 }  // namespace pccl

@@ -361,6 +361,78 @@ def test_gelu_forward_and_backward_with_bias_gradient(shape):
         torch.testing.assert_close(gb.float(), want, rtol=1e-2, atol=1e-2 * float(want.abs().max()) + 1e-3)
 
 
+@pytest.mark.parametrize("captured", [False, True], ids=["stream", "graph"])
+@pytest.mark.parametrize("T", [40, 1000, 4096])
+def test_chain_of_early_launches_equals_one_at_a_time(T, captured):
+    """Kernels may take their places before the one in front of them has ended: a chain in which each reads what
+    the last wrote, writes over what it read and shares its scratch, against the same chain with a wait behind every call,
+    on a stream and from a graph that is replayed."""
+    import pccl
+
+    C = pccl._C
+    g = torch.Generator(device=DEV).manual_seed(T)
+    d = 1024
+
+    def rnd(*shape, std=1.0):
+        return (torch.randn(*shape, device=DEV, generator=g) * std).to(torch.bfloat16)
+
+    x0, b0 = rnd(T, d), rnd(T, d)
+    w1, bias, w2 = rnd(2048, d, std=0.03), rnd(2048), rnd(d, 2048, std=0.03)
+    gam, bet = rnd(d, std=0.02) + 1, rnd(d, std=0.02)
+    tgt = torch.randint(0, 2048, (T,), device=DEV, generator=g)
+    x, b = torch.empty_like(x0), torch.empty_like(b0)
+    gw, gb, sums, cols = (torch.empty(d, device=DEV, dtype=torch.bfloat16) for _ in range(4))
+    loss, norm = torch.zeros(1, device=DEV), torch.zeros(1, device=DEV)
+    state = [torch.zeros(T * d, device=DEV) for _ in range(3)]
+    param = torch.zeros(T * d, device=DEV, dtype=torch.bfloat16)
+
+    def chain(pause):
+        out = []
+        x.copy_(x0), b.copy_(b0), loss.zero_(), norm.zero_()
+        for s in state:
+            s.zero_()
+        steps = [
+            lambda: C.ln_fwd(x, b, gam, bet, 1e-5),
+            lambda: C.gemm_ex(out[0][0], w1, False, False, bias, None, None),
+            lambda: C.ce_fwd_bwd(out[1], tgt, loss, 1.0 / T, -100),
+            lambda: C.gemm_ex(out[1], w2, False, False, None, x, None),
+            lambda: C.ln_bwd(x, b, out[0][1], out[0][2], gam, gw, gb, x, sums),
+            lambda: C.col_sum(out[4], cols),
+            lambda: C.gelu(out[4]),
+            lambda: C.gemm_ex(out[6], w2, False, True, None, out[1], None),
+            lambda: C.sq_norm(out[4], norm),
+            lambda: C.adamw(state[0], state[1], state[2], out[4].view(-1), param, 1e-3, 0.9, 0.95, 1e-8, 0.1, 1, 1.0, 1.0, norm),
+        ]
+        for s in steps:
+            out.append(s())
+            if pause:
+                torch.cuda.synchronize()
+        return [out[0][0], out[1], x, b, out[4], out[6], gw, gb, sums, cols, param, state[0]]
+
+    want = [t.clone() for t in chain(True)]
+    if captured:
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            chain(False)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = chain(False)
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+    else:
+        for _ in range(5):
+            got = chain(False)
+        torch.cuda.synchronize()
+    names = ["y", "hidden", "x", "stream", "dx", "gelu", "gw", "gb", "sums", "cols", "param", "master"]
+    for n, a, e in zip(names, got, want):
+        if n in ("param", "master"):        # the order of the norm's partial sums is free
+            torch.testing.assert_close(a.float(), e.float(), rtol=1e-2, atol=1e-6)
+        else:
+            assert torch.equal(a, e), n
+
+
 @pytest.mark.parametrize("fused_gelu_gemm,overlap_wgrad,gelu_bwd_gemm",
                          [(False, False, False), (True, False, False), (False, True, False), (False, False, True)])
 def test_engine_fused_kernels_match_autograd_at_width_1024(fused_gelu_gemm, overlap_wgrad, gelu_bwd_gemm):
