@@ -58,6 +58,8 @@ bool g_dynamic_tiles = false;  // hand tiles out at run time instead of dealing 
 int g_max_pairs = 0, g_group_m = 0;      // tuning knobs, 0: the kernel's defaults
 int g_wide = -1;                         // units of two row-tiles that share their W half: 1 always, 0 never, -1 where measured faster
 
+constexpr long long kSplitCostNs = 6000;
+
 SkWorkspace& sk_workspace(int device, cudaStream_t stream, int pairs) {
   static std::map<std::pair<int, cudaStream_t>, SkWorkspace> all;
   static std::mutex mu;
@@ -117,6 +119,12 @@ void maybe_split_last_wave(GemmArgs& a, int device, cudaStream_t stream) {
   // fewer tiles than CTA pairs: splitting every tile wins a single cold launch, but back to back under the power
   // cap the unsplit launch is faster (2048 x 2048 x 8192: 65 against 74 us), so it is opt-in
   if ((long long)((a.M + 255) / 256) * ((a.N + 255) / 256) < sms / 2 && !g_split_single_round) return;
+  if (!g_split_single_round) {
+    // The split saves the idle part of the last round and costs the exchange of partial sums.  @@SKCOST@@
+    const long long G = sms / 2, T = (long long)((a.M + 255) / 256) * ((a.N + 255) / 256);
+    const long long rounds = (T + G - 1) / G, nkb = (a.K + 63) / 64;
+    if (281 * nkb * (rounds * G - T) / G < kSplitCostNs) return;
+  }
   SkWorkspace& w = sk_workspace(device, stream, sms / 2);
   a.sk_tiles = n;
   a.sk_scratch = w.scratch.data_ptr<float>();

@@ -51,8 +51,8 @@ cudaError_t launch_ln_fwd(const void* x, void* branch, const void* gamma, const 
 
 // Layer-norm backward for bf16 activations with d in {1024, 2048, 4096}: writes dx (+ resid when
 // given), dgamma, dbeta and, when dx_col_sum is given, the column sums of the stored dx.
-// scratch: 3 * ln_bwd_blocks() * d floats.
-int ln_bwd_blocks();
+// scratch: 3 * ln_bwd_blocks(d) * d floats.
+int ln_bwd_blocks(int d);
 cudaError_t launch_ln_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const void* gamma, void* dx,
                           const void* resid, void* dgamma, void* dbeta, void* dx_col_sum, float* scratch, int64_t T, int d,
                           cudaStream_t s);

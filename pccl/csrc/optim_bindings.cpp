@@ -231,7 +231,7 @@ at::Tensor ln_bwd(const at::Tensor& dy, const at::Tensor& x, const at::Tensor& m
   c10::cuda::CUDAGuard guard(dy.device());
   const int dev = dy.get_device();
   at::Tensor dx = at::empty_like(dy);
-  const int64_t part = (int64_t)ln_bwd_blocks() * d;
+  const int64_t part = (int64_t)ln_bwd_blocks((int)d) * d;
   at::Tensor& sc = scratch(dev, 3 * part + (int64_t)64 * 8192);
   float* pg = sc.data_ptr<float>() + (int64_t)64 * 8192;     // the front of the buffer belongs to col_sum
   PCCL_CUDA(launch_ln_bwd(dy.data_ptr(), x.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr(),

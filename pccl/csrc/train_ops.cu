@@ -17,26 +17,6 @@ namespace pccl {
 
 namespace {
 
-__device__ __forceinline__ void unpack8(const uint4& q, float* f) {
-  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __uint_as_float(w[i] << 16);
-    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-  }
-}
-__device__ __forceinline__ uint4 pack8(const float* f) {
-  uint32_t w[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-    w[i] = *reinterpret_cast<uint32_t*>(&h);
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-__device__ __forceinline__ float round_bf16(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
-
 // ---------------------------------------------------------------- column sum
 // out[c] = sum_r X[r, c]; X is [T, N] bf16 row-major with N % 8 == 0.  A block covers 256
 // columns (a warp reads 512 contiguous bytes of one row) in eight row lanes, one per warp, and one slice of the
@@ -175,261 +155,129 @@ __global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* __
 
 // ---------------------------------------------------------------- layer-norm backward
 // One pass over dy and x:  dx = rstd * (g - mean(g) - xhat * mean(g * xhat)),  g = dy * gamma,
-// and per-block partial sums of dgamma = sum_r dy * xhat, dbeta = sum_r dy.
+// and per-block partial sums of dgamma = sum_r dy * xhat, dbeta = sum_r dy.  With `resid` the gradient that
+// flows around the layer norm (the residual connection) is added to dx in the same pass (in fp32, before the one
+// rounding); with `pdx` the kernel also sums the columns of dx (the bias gradient of the linear layer whose output
+// gradient dx is).  A block leaves one partial row per array, and a second small kernel adds the blocks' partials.
 //
-// 128 threads work on one row (EPT = d / 128 elements each, in 16-byte vectors).  A block has
-// two such row groups and each group takes RB rows per iteration: all their loads (dy, x and the
-// residual gradient, kept packed as bf16) are issued before the first use, so a block keeps
-// 2 * RB rows in flight, and the RB row reductions share one pair of block barriers.
-// With `resid` the gradient that flows around the layer norm (the residual connection) is added
-// to dx in the same pass (in fp32, before the one rounding); with `pdx` the kernel also sums the columns of dx (the
-// bias gradient of the linear layer whose output gradient dx is).  The two groups add their
-// column sums through shared memory, so a block leaves one partial row per array, and a second
-// small kernel adds the blocks' partials.
-template <int EPT>
-__device__ __forceinline__ void ln_bwd_combine(const float* acc, float* comb, float* out_row, int rg, int t) {
-  constexpr int NV = EPT / 8;
-  if (rg == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      float4* c = reinterpret_cast<float4*>(comb + (t + 128 * k) * 8);
-      c[0] = make_float4(acc[8 * k], acc[8 * k + 1], acc[8 * k + 2], acc[8 * k + 3]);
-      c[1] = make_float4(acc[8 * k + 4], acc[8 * k + 5], acc[8 * k + 6], acc[8 * k + 7]);
-    }
-  }
-  __syncthreads();
-  if (rg == 1) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      const float4* c = reinterpret_cast<const float4*>(comb + (t + 128 * k) * 8);
-      const float4 a0 = c[0], a1 = c[1];
-      float4* o = reinterpret_cast<float4*>(out_row + (t + 128 * k) * 8);
-      o[0] = make_float4(a0.x + acc[8 * k], a0.y + acc[8 * k + 1], a0.z + acc[8 * k + 2], a0.w + acc[8 * k + 3]);
-      o[1] = make_float4(a1.x + acc[8 * k + 4], a1.y + acc[8 * k + 5], a1.z + acc[8 * k + 6], a1.w + acc[8 * k + 7]);
-    }
-  }
-  __syncthreads();
-}
-
-template <int EPT, int RB>
-__global__ void __launch_bounds__(256, 1)
+// D / 8 threads work on one row (one 16-byte vector each), so the three column accumulators take 24 registers and
+// 16 warps of 128 registers fit on an SM for every width.  A block takes two rows at a time, and the loads of
+// the next two are issued before the reductions of the current ones: with one buffer of four rows instead, the memory
+// system waits while the block reduces.  One barrier per two rows (the row sums are double-buffered); the
+// arithmetic goes two elements per instruction.  Bound by HBM at many rows, by the chain of row reductions at few.
+// Measured with residual and column sums, without the kernel that adds the partials: @@LNB@@.
+template <int D, int RB>
+__global__ void __launch_bounds__(D / 8, 4096 / D)
     ln_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean,
-                  const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma,
-                  const __nv_bfloat16* __restrict__ resid, __nv_bfloat16* __restrict__ dx, float* __restrict__ pgamma,
-                  float* __restrict__ pbeta, float* __restrict__ pdx, int64_t T, int d) {
-  constexpr int NV = EPT / 8;
-  __shared__ float red[2][RB][4][2];
-  __shared__ __align__(16) float comb[128 * EPT];
+                  const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ resid,
+                  __nv_bfloat16* __restrict__ dx, float* __restrict__ pgamma, float* __restrict__ pbeta, float* __restrict__ pdx,
+                  int64_t T) {
   pdl_wait();
   pdl_trigger();
-  const int rg = threadIdx.x >> 7, t = threadIdx.x & 127, warp_in_rg = t >> 5, lane = t & 31;
-  uint4 pgam[NV];
-  float dgam[EPT], dbet[EPT], dxs[EPT];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    pgam[k] = *reinterpret_cast<const uint4*>(gamma + (t + 128 * k) * 8);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) dgam[8 * k + e] = dbet[8 * k + e] = dxs[8 * k + e] = 0.f;
-  }
-  const float inv_d = 1.0f / (float)d;
-  const int64_t step = 2 * RB * (int64_t)gridDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * 2 * RB; base < T; base += step) {
-    uint4 pdy[RB][NV], px[RB][NV], pr[RB][NV];
-    float mu[RB], rs[RB];
-    // ---- all loads of this group's rows
-#pragma unroll
-    for (int j = 0; j < RB; ++j) {
-      const int64_t r = base + rg * RB + j;
-      mu[j] = 0.f;
-      rs[j] = 0.f;
-#pragma unroll
-      for (int k = 0; k < NV; ++k) pdy[j][k] = px[j][k] = pr[j][k] = make_uint4(0, 0, 0, 0);
-      if (r < T) {
-        mu[j] = mean[r];
-        rs[j] = rstd[r];
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-          const int64_t off = r * d + (t + 128 * k) * 8;
-          pdy[j][k] = *reinterpret_cast<const uint4*>(dy + off);
-          px[j][k] = *reinterpret_cast<const uint4*>(x + off);
-          if (resid != nullptr) pr[j][k] = *reinterpret_cast<const uint4*>(resid + off);
-        }
-      }
-    }
-    // ---- row sums and the weight/bias gradient sums (rows past the end hold zeros)
-#pragma unroll
-    for (int j = 0; j < RB; ++j) {
-      float s1 = 0.f, s2 = 0.f;
-      const float nmr = -mu[j] * rs[j];
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        float a[8], b[8], g[8];
-        unpack8(pdy[j][k], a);
-        unpack8(px[j][k], b);
-        unpack8(pgam[k], g);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float xhat = fmaf(b[e], rs[j], nmr);
-          const float gg = a[e] * g[e];
-          s1 += gg;
-          s2 = fmaf(gg, xhat, s2);
-          dgam[8 * k + e] = fmaf(a[e], xhat, dgam[8 * k + e]);
-          dbet[8 * k + e] += a[e];
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      }
-      if (lane == 0) {
-        red[rg][j][warp_in_rg][0] = s1;
-        red[rg][j][warp_in_rg][1] = s2;
-      }
-    }
-    __syncthreads();
-    // ---- dx
-#pragma unroll
-    for (int j = 0; j < RB; ++j) {
-      const int64_t r = base + rg * RB + j;
-      if (r < T) {
-        const float m1 = (red[rg][j][0][0] + red[rg][j][1][0] + red[rg][j][2][0] + red[rg][j][3][0]) * inv_d;
-        const float m2 = (red[rg][j][0][1] + red[rg][j][1][1] + red[rg][j][2][1] + red[rg][j][3][1]) * inv_d;
-        // dx = rs * (dy * gamma - m1 - xhat * m2) = dy * (gamma * rs) - x * c2 + c0
-        const float c2 = rs[j] * rs[j] * m2;
-        const float c0 = fmaf(mu[j], c2, -m1 * rs[j]);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-          float a[8], b[8], g[8], o8[8];
-          unpack8(pdy[j][k], a);
-          unpack8(px[j][k], b);
-          unpack8(pgam[k], g);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o8[e] = fmaf(a[e], g[e] * rs[j], fmaf(b[e], -c2, c0));
-          if (resid != nullptr) {
-            float q8[8];
-            unpack8(pr[j][k], q8);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o8[e] += q8[e];                        // one rounding, at the store
-          }
-          *reinterpret_cast<uint4*>(dx + r * d + (t + 128 * k) * 8) = pack8(o8);
-          if (pdx != nullptr) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) dxs[8 * k + e] += o8[e];
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  ln_bwd_combine<EPT>(dgam, comb, pgamma + (int64_t)blockIdx.x * d, rg, t);
-  ln_bwd_combine<EPT>(dbet, comb, pbeta + (int64_t)blockIdx.x * d, rg, t);
-  if (pdx != nullptr) ln_bwd_combine<EPT>(dxs, comb, pdx + (int64_t)blockIdx.x * d, rg, t);
-}
-
-// The d = 2048 form: all 256 threads of a block work on one row (8 elements each), RB rows per
-// iteration, two blocks per SM.  The column accumulators then take 24 registers instead of 48, so
-// four rows of loads fit beside them in 128 registers; two resident blocks overlap one block's
-// loads with the other's arithmetic (measured 1.2x faster than the two-group form at 8192 rows, 1.4x at 32768).
-template <int RB>
-__global__ void __launch_bounds__(256, 2)
-    ln_bwd_row256_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                         const float* __restrict__ mean, const float* __restrict__ rstd,
-                         const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ resid,
-                         __nv_bfloat16* __restrict__ dx, float* __restrict__ pgamma, float* __restrict__ pbeta,
-                         float* __restrict__ pdx, int64_t T) {
-  pdl_wait();
-  pdl_trigger();
-  constexpr int d = 2048;
-  __shared__ float red[RB][8][2];
+  constexpr int NW = D / 256;
+  __shared__ float2 red[2][RB][NW];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  float g[8], dgam[8], dbet[8], dxs[8];
-  unpack8(*reinterpret_cast<const uint4*>(gamma + t * 8), g);
+  F2 g[4], dgam[4], dbet[4], dxs[4];
+  {
+    const uint4 q = *reinterpret_cast<const uint4*>(gamma + t * 8);
+    g[0] = unpack2(q.x), g[1] = unpack2(q.y), g[2] = unpack2(q.z), g[3] = unpack2(q.w);
+  }
 #pragma unroll
-  for (int e = 0; e < 8; ++e) dgam[e] = dbet[e] = dxs[e] = 0.f;
-  const float inv_d = 1.0f / (float)d;
-  const int64_t step = (int64_t)RB * gridDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * RB; base < T; base += step) {
-    uint4 pdy[RB], px[RB], pr[RB];
+  for (int e = 0; e < 4; ++e) dgam[e] = dbet[e] = dxs[e] = f2(0.f);
+  struct Rows {
+    uint4 dy[RB], x[RB], r[RB];
     float mu[RB], rs[RB];
+  };
+  auto load = [&](Rows& b, int64_t base) {                  // rows past the end hold zeros
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
       const int64_t r = base + j;
-      mu[j] = rs[j] = 0.f;
-      pdy[j] = px[j] = pr[j] = make_uint4(0, 0, 0, 0);
+      b.mu[j] = b.rs[j] = 0.f;
+      b.dy[j] = b.x[j] = b.r[j] = make_uint4(0, 0, 0, 0);
       if (r < T) {
-        const int64_t off = r * d + t * 8;
-        mu[j] = mean[r];
-        rs[j] = rstd[r];
-        pdy[j] = *reinterpret_cast<const uint4*>(dy + off);
-        px[j] = *reinterpret_cast<const uint4*>(x + off);
-        if (resid != nullptr) pr[j] = *reinterpret_cast<const uint4*>(resid + off);
+        const int64_t off = r * D + t * 8;
+        b.dy[j] = *reinterpret_cast<const uint4*>(dy + off);
+        b.x[j] = *reinterpret_cast<const uint4*>(x + off);
+        if (resid != nullptr) b.r[j] = *reinterpret_cast<const uint4*>(resid + off);
+        b.mu[j] = mean[r];
+        b.rs[j] = rstd[r];
       }
     }
+  };
+  constexpr float inv_d = 1.0f / (float)D;
+  const int64_t step = (int64_t)RB * gridDim.x;
+  Rows cur, nxt;
+  load(cur, (int64_t)blockIdx.x * RB);
+  int buf = 0;
+  for (int64_t base = (int64_t)blockIdx.x * RB; base < T; base += step, buf ^= 1) {
+    load(nxt, base + step);
+    // ---- row sums and the weight/bias gradient sums
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
-      float s1 = 0.f, s2 = 0.f, a[8], b[8];
-      const float nmr = -mu[j] * rs[j];
-      unpack8(pdy[j], a);
-      unpack8(px[j], b);
+      const uint32_t aw[4] = {cur.dy[j].x, cur.dy[j].y, cur.dy[j].z, cur.dy[j].w}, bw[4] = {cur.x[j].x, cur.x[j].y, cur.x[j].z, cur.x[j].w};
+      const F2 rs = f2(cur.rs[j]), nmr = f2(-cur.mu[j] * cur.rs[j]);
+      F2 t1 = f2(0.f), t2 = f2(0.f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float xhat = fmaf(b[e], rs[j], nmr);
-        const float gg = a[e] * g[e];
-        s1 += gg;
-        s2 = fmaf(gg, xhat, s2);
-        dgam[e] = fmaf(a[e], xhat, dgam[e]);
-        dbet[e] += a[e];
+      for (int e = 0; e < 4; ++e) {
+        const F2 a = unpack2(aw[e]), xhat = fma2(unpack2(bw[e]), rs, nmr), gg = a * g[e];
+        t1 = t1 + gg;
+        t2 = fma2(gg, xhat, t2);
+        dgam[e] = fma2(a, xhat, dgam[e]);
+        dbet[e] = dbet[e] + a;
       }
+      float s1, s2, hi;
+      split(t1, s1, hi);
+      s1 += hi;
+      split(t2, s2, hi);
+      s2 += hi;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
         s2 += __shfl_xor_sync(0xffffffffu, s2, o);
       }
-      if (lane == 0) {
-        red[j][warp][0] = s1;
-        red[j][warp][1] = s2;
-      }
+      if (lane == 0) red[buf][j][warp] = make_float2(s1, s2);
     }
     __syncthreads();
+    // ---- dx = rs * (dy * gamma - m1 - xhat * m2) = dy * (gamma * rs) - x * c2 + c0
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
       const int64_t r = base + j;
       if (r < T) {
         float m1 = 0.f, m2 = 0.f;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) {
-          m1 += red[j][w][0];
-          m2 += red[j][w][1];
+        for (int w = 0; w < NW; ++w) {
+          m1 += red[buf][j][w].x;
+          m2 += red[buf][j][w].y;
         }
         m1 *= inv_d;
         m2 *= inv_d;
-        const float c2 = rs[j] * rs[j] * m2;
-        const float c0 = fmaf(mu[j], c2, -m1 * rs[j]);
-        float a[8], b[8], o8[8];
-        unpack8(pdy[j], a);
-        unpack8(px[j], b);
+        const float c2 = cur.rs[j] * cur.rs[j] * m2;
+        const F2 c0 = f2(fmaf(cur.mu[j], c2, -m1 * cur.rs[j])), nc2 = f2(-c2), rs = f2(cur.rs[j]);
+        const uint32_t aw[4] = {cur.dy[j].x, cur.dy[j].y, cur.dy[j].z, cur.dy[j].w}, bw[4] = {cur.x[j].x, cur.x[j].y, cur.x[j].z, cur.x[j].w};
+        const uint32_t qw[4] = {cur.r[j].x, cur.r[j].y, cur.r[j].z, cur.r[j].w};
+        uint32_t ow[4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o8[e] = fmaf(a[e], g[e] * rs[j], fmaf(b[e], -c2, c0));
-        if (resid != nullptr) {
-          float q8[8];
-          unpack8(pr[j], q8);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o8[e] += q8[e];                          // one rounding, at the store
+        for (int e = 0; e < 4; ++e) {
+          F2 o = fma2(unpack2(aw[e]), g[e] * rs, fma2(unpack2(bw[e]), nc2, c0));
+          if (resid != nullptr) o = o + unpack2(qw[e]);                        // one rounding, at the store
+          dxs[e] = dxs[e] + o;
+          float lo, hi;
+          split(o, lo, hi);
+          const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+          ow[e] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        *reinterpret_cast<uint4*>(dx + r * d + t * 8) = pack8(o8);
-        if (pdx != nullptr) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) dxs[e] += o8[e];
-        }
+        *reinterpret_cast<uint4*>(dx + r * D + t * 8) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
       }
     }
-    __syncthreads();
+    cur = nxt;
   }
-  auto put = [&](float* row, const float* acc) {
-    float4* o = reinterpret_cast<float4*>(row + (int64_t)blockIdx.x * d + t * 8);
-    o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  auto put = [&](float* row, const F2 (&acc)[4]) {
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split(acc[e], v[2 * e], v[2 * e + 1]);
+    float4* o = reinterpret_cast<float4*>(row + (int64_t)blockIdx.x * D + t * 8);
+    o[0] = make_float4(v[0], v[1], v[2], v[3]);
+    o[1] = make_float4(v[4], v[5], v[6], v[7]);
   };
   put(pgamma, dgam);
   put(pbeta, dbet);
@@ -437,38 +285,34 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // Adds the per-block partial sums of up to three arrays (blockIdx.y picks the array): a block
-// owns 32 columns, its 8 warps split the partials.
+// owns 32 columns, its 32 warps split the partials and keep four rows in flight each (up to 592 rows: five
+// rounds; with 8 warps the rounds were what this kernel took).
 struct LnBwdFinalizeArgs {
   const float* part[3];
   __nv_bfloat16* out[3];
 };
 
-__global__ void __launch_bounds__(256) ln_bwd_finalize_kernel(LnBwdFinalizeArgs f, int nparts, int d) {
-  __shared__ float sa[8][33];
+__global__ void __launch_bounds__(1024) ln_bwd_finalize_kernel(LnBwdFinalizeArgs f, int nparts, int d) {
   pdl_wait();
   pdl_trigger();
+  __shared__ float sa[32][33];
   const float* __restrict__ part = f.part[blockIdx.y];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+  const int c = blockIdx.x * 32 + lane;                // d is a multiple of 32
   float a = 0.f;
-  if (c < d) {
-    int p = w;
-    for (; p + 56 < nparts; p += 64) {              // eight rows in flight
-      float va[8];
+  for (int p = w; p < nparts; p += 128) {
+    float v[4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) va[k] = __ldcg(part + (int64_t)(p + 8 * k) * d + c);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) a += va[k];
-    }
-    for (; p < nparts; p += 8) a += __ldcg(part + (int64_t)p * d + c);
+    for (int k = 0; k < 4; ++k) v[k] = p + 32 * k < nparts ? __ldcg(part + (int64_t)(p + 32 * k) * d + c) : 0.f;
+    a += (v[0] + v[1]) + (v[2] + v[3]);
   }
   sa[w][lane] = a;
   __syncthreads();
-  if (w == 0 && c < d) {
+  // warp w adds column w's 32 sums
+  a = sa[lane][w];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) a += sa[k][lane];
-    f.out[blockIdx.y][c] = __float2bfloat16_rn(a);
-  }
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if (lane == 0) f.out[blockIdx.y][blockIdx.x * 32 + w] = __float2bfloat16_rn(a);
 }
 
 // ---------------------------------------------------------------- GELU forward
@@ -500,71 +344,110 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__
 }
 
 // ---------------------------------------------------------------- residual add + layer norm
-// One row per 128-thread block iteration.  With `branch` the row is x + branch, rounded to
-// bf16 and written back over `branch` (it becomes the new residual stream); the statistics and
-// the normalised output are taken from the rounded values, which is what the backward pass
-// reads.  Writes y = (v - mean) * rstd * gamma + beta, mean and rstd (biased variance).
-__device__ __forceinline__ float block_sum_128(float s, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  s = red[0] + red[1] + red[2] + red[3];
-  __syncthreads();
-  return s;
-}
-
-template <int EPT>
-__global__ void __launch_bounds__(128) ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* branch,
-                                                     const __nv_bfloat16* __restrict__ gamma,
-                                                     const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
-                                                     float* __restrict__ mean, float* __restrict__ rstd, int64_t T, int d,
-                                                     float eps) {
-  constexpr int NV = EPT / 8;
-  __shared__ float red[4];
+// With `branch` the row is x + branch, rounded to bf16 and written back over `branch` (it becomes the new residual
+// stream); the statistics and the normalised output are taken from the rounded values, which is what the
+// backward pass reads.  Writes y = (v - mean) * rstd * gamma + beta, mean and rstd (biased variance, from the
+// deviations).
+//
+// A warp works on one row (two warps for 4096 columns) and keeps it as it is stored, eight 16-byte vectors per
+// lane: all its loads are in flight at once, the row sums need no block barrier, and the packed row takes 32 registers.
+// Bound by HBM.  Measured with branch against 128 threads per row, fp32 in registers and four barriers:
+// @@LNF@@.
+constexpr int kLnFwdWarps = 4;      // per block: small ones, so that few rows still reach every SM
+template <int D>
+__global__ void __launch_bounds__(32 * kLnFwdWarps, 6) ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* branch,
+                                                        const __nv_bfloat16* __restrict__ gamma,
+                                                        const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
+                                                        float* __restrict__ mean, float* __restrict__ rstd, int64_t T, float eps) {
   pdl_wait();
   pdl_trigger();
-  const int t = threadIdx.x;
-  const float inv_d = 1.0f / (float)d;
-  for (int64_t r = blockIdx.x; r < T; r += gridDim.x) {
-    float v[EPT];
-    float s = 0.f;
+  constexpr int WPR = D > 2048 ? 2 : 1;                // warps per row
+  constexpr int NV = D / (256 * WPR);                  // vectors per lane
+  __shared__ float part[2][kLnFwdWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t r = ((int64_t)blockIdx.x * kLnFwdWarps + warp) / WPR;
+  const bool live = r < T;                             // a block's last rows may not exist (the block meets at barriers if WPR > 1)
+  const int c0 = ((warp % WPR) * 32 + lane) * 8;       // first column of vector k: c0 + k * 256 * WPR
+  constexpr float inv_d = 1.0f / (float)D;
+  uint4 v[NV];
+  float s = 0.f;
+  if (live) {
+    const int64_t off = r * D + c0;
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      const int64_t off = r * d + (t + 128 * k) * 8;
-      unpack8(*reinterpret_cast<const uint4*>(x + off), v + 8 * k);
-      if (branch != nullptr) {
-        float b[8];
-        unpack8(*reinterpret_cast<const uint4*>(branch + off), b);
+    for (int k = 0; k < NV; ++k) v[k] = *reinterpret_cast<const uint4*>(x + off + k * 256 * WPR);
+    if (branch != nullptr) {
+      uint4 b[NV];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[8 * k + e] = round_bf16(v[8 * k + e] + b[e]);
-        *reinterpret_cast<uint4*>(branch + off) = pack8(v + 8 * k);
+      for (int k = 0; k < NV; ++k) b[k] = *reinterpret_cast<const uint4*>(branch + off + k * 256 * WPR);
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        uint32_t vw[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+        const uint32_t bw[4] = {b[k].x, b[k].y, b[k].z, b[k].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float lo, hi;
+          split(unpack2(vw[e]) + unpack2(bw[e]), lo, hi);
+          const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+          vw[e] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        v[k] = make_uint4(vw[0], vw[1], vw[2], vw[3]);
+        *reinterpret_cast<uint4*>(branch + off + k * 256 * WPR) = v[k];
       }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) s += v[8 * k + e];
     }
-    const float mu = block_sum_128(s, red) * inv_d;
-    float s2 = 0.f;
+    F2 a = f2(0.f);
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      const float c = v[i] - mu;
-      s2 += c * c;
+    for (int k = 0; k < NV; ++k) a = a + ((unpack2(v[k].x) + unpack2(v[k].y)) + (unpack2(v[k].z) + unpack2(v[k].w)));
+    float hi;
+    split(a, s, hi);
+    s += hi;
+  }
+  auto row_sum = [&](float a, int which) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (WPR > 1) {
+      if (lane == 0) part[which][warp] = a;
+      __syncthreads();
+      a = part[which][warp & ~1] + part[which][warp | 1];
     }
-    const float rs = rsqrtf(block_sum_128(s2, red) * inv_d + eps);
+    return a;
+  };
+  const float mu = row_sum(s, 0) * inv_d;
+  F2 dev = f2(0.f);
+  const F2 nmu = f2(-mu);
+  if (live) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const int c0 = (t + 128 * k) * 8;
-      float g[8], b[8], o[8];
-      unpack8(*reinterpret_cast<const uint4*>(gamma + c0), g);
-      unpack8(*reinterpret_cast<const uint4*>(beta + c0), b);
+      const uint32_t vw[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = (v[8 * k + e] - mu) * rs * g[e] + b[e];
-      *reinterpret_cast<uint4*>(y + r * d + c0) = pack8(o);
+      for (int e = 0; e < 4; ++e) {
+        const F2 c = unpack2(vw[e]) + nmu;
+        dev = fma2(c, c, dev);
+      }
     }
-    if (t == 0) {
-      mean[r] = mu;
-      rstd[r] = rs;
+  }
+  float s2, hi2;
+  split(dev, s2, hi2);
+  const float rs = rsqrtf(row_sum(s2 + hi2, 1) * inv_d + eps);
+  if (!live) return;
+  const F2 rs2 = f2(rs);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int c = c0 + k * 256 * WPR;
+    const uint4 gq = *reinterpret_cast<const uint4*>(gamma + c), bq = *reinterpret_cast<const uint4*>(beta + c);
+    const uint32_t vw[4] = {v[k].x, v[k].y, v[k].z, v[k].w}, gw[4] = {gq.x, gq.y, gq.z, gq.w}, bw[4] = {bq.x, bq.y, bq.z, bq.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float lo, hi;
+      split(fma2((unpack2(vw[e]) + nmu) * rs2, unpack2(gw[e]), unpack2(bw[e])), lo, hi);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+      o[e] = *reinterpret_cast<const uint32_t*>(&h);
     }
+    *reinterpret_cast<uint4*>(y + r * D + c) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  if (lane == 0 && warp % WPR == 0) {
+    mean[r] = mu;
+    rstd[r] = rs;
   }
 }
 
@@ -619,7 +502,7 @@ cudaError_t launch_gelu_fwd(const void* in, void* out, int64_t n, cudaStream_t s
 cudaError_t launch_ln_fwd(const void* x, void* branch, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                           int64_t T, int d, float eps, cudaStream_t s) {
   if (T <= 0) return cudaSuccess;
-  int64_t blocks = T < 148 * 8 ? T : 148 * 8;
+  const int64_t blocks = (T * (d > 2048 ? 2 : 1) + kLnFwdWarps - 1) / kLnFwdWarps;
   auto* X = (const __nv_bfloat16*)x;
   auto* B = (__nv_bfloat16*)branch;
   auto* G = (const __nv_bfloat16*)gamma;
@@ -627,46 +510,43 @@ cudaError_t launch_ln_fwd(const void* x, void* branch, const void* gamma, const 
   auto* Y = (__nv_bfloat16*)y;
   cudaError_t e = cudaSuccess;
   switch (d / 128) {
-    case 8: e = launch_pdl(ln_fwd_kernel<8>, (int)blocks, 128, 0, s, X, B, G, Be, Y, mean, rstd, T, d, eps); break;
-    case 16: e = launch_pdl(ln_fwd_kernel<16>, (int)blocks, 128, 0, s, X, B, G, Be, Y, mean, rstd, T, d, eps); break;
-    case 32: e = launch_pdl(ln_fwd_kernel<32>, (int)blocks, 128, 0, s, X, B, G, Be, Y, mean, rstd, T, d, eps); break;
+    case 8: e = launch_pdl(ln_fwd_kernel<1024>, (unsigned)blocks, 32 * kLnFwdWarps, 0, s, X, B, G, Be, Y, mean, rstd, T, eps); break;
+    case 16: e = launch_pdl(ln_fwd_kernel<2048>, (unsigned)blocks, 32 * kLnFwdWarps, 0, s, X, B, G, Be, Y, mean, rstd, T, eps); break;
+    case 32: e = launch_pdl(ln_fwd_kernel<4096>, (unsigned)blocks, 32 * kLnFwdWarps, 0, s, X, B, G, Be, Y, mean, rstd, T, eps); break;
     default: return cudaErrorInvalidValue;
   }
   return e;
 }
 
-int ln_bwd_blocks() { return 296; }      // at most two blocks per SM; each leaves one partial row per array
+// Blocks of the widest grid: 4096 / d per SM, each leaves one partial row of d floats per array.
+int ln_bwd_blocks(int d) { return 148 * (4096 / d); }
 
 cudaError_t launch_ln_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const void* gamma, void* dx,
                           const void* resid, void* dgamma, void* dbeta, void* dx_col_sum, float* scratch, int64_t T, int d,
                           cudaStream_t s) {
   if (T <= 0) return cudaSuccess;
-  // d = 2048: one row per 256 threads, four rows per iteration, two blocks per SM; other widths: two
-  // row groups of 128 threads per block, one block per SM, rows per group limited by registers
-  const bool row256 = d == 2048;
-  const int rows_per_iter = row256 ? 4 : 2 * (d <= 2048 ? 4 : 1);
-  int blocks = row256 ? ln_bwd_blocks() : 148;
-  if ((int64_t)blocks * rows_per_iter > T) blocks = (int)((T + rows_per_iter - 1) / rows_per_iter);
+  int blocks = ln_bwd_blocks(d);
+  if ((int64_t)blocks * 2 > T) blocks = (int)((T + 1) / 2);                 // two rows per block and iteration
   auto* DY = (const __nv_bfloat16*)dy;
   auto* X = (const __nv_bfloat16*)x;
   auto* G = (const __nv_bfloat16*)gamma;
   auto* RS = (const __nv_bfloat16*)resid;
   auto* DX = (__nv_bfloat16*)dx;
   float* pgamma = scratch;
-  float* pbeta = scratch + (int64_t)ln_bwd_blocks() * d;
-  float* pdx = dx_col_sum != nullptr ? scratch + 2 * (int64_t)ln_bwd_blocks() * d : nullptr;
+  float* pbeta = scratch + (int64_t)ln_bwd_blocks(d) * d;
+  float* pdx = dx_col_sum != nullptr ? scratch + 2 * (int64_t)ln_bwd_blocks(d) * d : nullptr;
   cudaError_t e = cudaSuccess;
   switch (d / 128) {
-    case 8: e = launch_pdl(ln_bwd_kernel<8, 4>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T, d); break;
-    case 16: e = launch_pdl(ln_bwd_row256_kernel<4>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
-    case 32: e = launch_pdl(ln_bwd_kernel<32, 1>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T, d); break;
+    case 8: e = launch_pdl(ln_bwd_kernel<1024, 2>, blocks, 128, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
+    case 16: e = launch_pdl(ln_bwd_kernel<2048, 2>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
+    case 32: e = launch_pdl(ln_bwd_kernel<4096, 2>, blocks, 512, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
     default: return cudaErrorInvalidValue;
   }
   if (e != cudaSuccess) return e;
   LnBwdFinalizeArgs f;
   f.part[0] = pgamma, f.part[1] = pbeta, f.part[2] = pdx;
   f.out[0] = (__nv_bfloat16*)dgamma, f.out[1] = (__nv_bfloat16*)dbeta, f.out[2] = (__nv_bfloat16*)dx_col_sum;
-  return launch_pdl(ln_bwd_finalize_kernel, dim3((d + 31) / 32, pdx != nullptr ? 3 : 2), 256, 0, s, f, blocks, d);
+  return launch_pdl(ln_bwd_finalize_kernel, dim3((d + 31) / 32, pdx != nullptr ? 3 : 2), 1024, 0, s, f, blocks, d);
 }
 
 }  // namespace pccl
