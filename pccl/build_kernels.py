@@ -50,6 +50,9 @@ SOURCES = [
     "comm.cpp",
     "segments.cpp",
     "collectives.cu",
+    "reduce_scatter_bf16.cu",
+    "reduce_scatter_f16.cu",
+    "reduce_scatter_f32.cu",
     "gemm_sm100.cu",
     "optim.cu",
     "train_ops.cu",
