@@ -388,15 +388,8 @@ void all_reduce(Comm& c, int gid, std::vector<at::Tensor> ts, int algo, int nlan
     // ring or both recursive; here one launch per chunk, in place (each rank's block of the sum
     // is formed in its own slot of the tensor and gathered from there).
     const uint64_t blk = n / (uint64_t)P;            // elements per rank
-    uint64_t cap = blk;
-    if (off < 0) {
-      // private tensors: partial sums and gathered blocks both pass through the staging area
-      cap = std::min(c.staging_bytes() / (uint64_t)(P - 1) / s, c.staging_bytes() / (uint64_t)P / s) / 8 * 8;
-      TORCH_CHECK(cap > 0, "staging area too small for an all-reduce");
-    } else {
-      cap = c.staging_bytes() / (uint64_t)(P - 1) / s / 8 * 8;   // the reduce-scatter phase stages partial sums
-      TORCH_CHECK(cap > 0, "staging area too small for an all-reduce");
-    }
+    const uint64_t cap = two_phase_staging(c.staging_bytes(), s, P, 0, off >= 0).cap;
+    TORCH_CHECK(cap > 0, "staging area too small for an all-reduce");
     for (uint64_t e0 = 0; e0 < blk; e0 += cap) {
       const uint64_t len = std::min(cap, blk - e0);
       AllReduceRsAgArgs a;
@@ -409,7 +402,8 @@ void all_reduce(Comm& c, int gid, std::vector<at::Tensor> ts, int algo, int nlan
       a.rs.out_sub_stride = blk * s;
       a.rs.stage_off = c.staging_off();
       a.rs.sub_elems = len;
-      a.rs.stage_elems = (len + 7) / 8 * 8;          // cap is a multiple of 8
+      const TwoPhaseStaging st = two_phase_staging(c.staging_bytes(), s, P, len, off >= 0);
+      a.rs.stage_elems = st.partial_stride;
       a.ag.nsub = 1;
       a.ag.sub_bytes = len * s;
       a.ag.in_sub_stride = blk * s;
@@ -432,7 +426,7 @@ void all_reduce(Comm& c, int gid, std::vector<at::Tensor> ts, int algo, int nlan
         a.ag.src_stride = blk * s;
       } else {
         a.ag.recv_off = c.staging_off();
-        a.ag.src_stride = cap * s;
+        a.ag.src_stride = st.gather_stride * s;
       }
       c.all_reduce_rsag(gid, a, nlanes, stream);
     }
@@ -670,6 +664,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rs_step", [](int algo, int P, int r, int t) { return step_tuple(rs_step(algo, P, r, t)); });
   m.def("rs_stage_offset", [](int algo, int P, int t) { return rs_stage_offset(algo, P, t); });
   m.def("rs_dep_mask", [](int algo, int P, int t) { return rs_dep_mask(algo, P, t); });
+  m.def("two_phase_staging", [](uint64_t staging_bytes, uint64_t elem_bytes, int P, uint64_t len, bool symmetric) {
+    const TwoPhaseStaging t = two_phase_staging(staging_bytes, elem_bytes, P, len, symmetric);
+    return std::make_tuple(t.cap, t.partial_stride, t.gather_stride);
+  }, "(elements per launch, distance of partial sums, distance of gathered blocks) of the two-phase all-reduce");
   m.def("slot_index", [](int lane, int kind, int src) { return slot_index(lane, kind, src); });
 
   py::class_<IpcSegment>(m, "IpcSegment")

@@ -142,6 +142,23 @@ PCCL_HD int rs_stage_offset(int algo, int P, int t) {
 // Total staging blocks an algorithm needs on every rank: P-1 for all of them.
 PCCL_HD int rs_stage_blocks(int /*algo*/, int P) { return P > 0 ? P - 1 : 0; }
 
+// Staging of the two-phase all-reduce, in elements: what one launch takes of each rank's block (cap, a multiple of 8),
+// and the distance between staged partial sums (phase one) and between gathered blocks (phase two).  Lanes are
+// not synchronised with one another, so a lane may be in phase two while another still reads its partial sums.  Where both
+// phases pass through the staging area (private tensors) the two distances are therefore the same: a lane's range
+// of slot k is then the same in both phases, whatever the length of this launch.  Symmetric tensors are gathered in place;
+// their partial sums lie as close as 16-byte boundaries allow.
+struct TwoPhaseStaging {
+  uint64_t cap, partial_stride, gather_stride;
+};
+PCCL_HD TwoPhaseStaging two_phase_staging(uint64_t staging_bytes, uint64_t elem_bytes, int P, uint64_t len, bool symmetric) {
+  TwoPhaseStaging t;
+  t.cap = staging_bytes / (uint64_t)(symmetric ? P - 1 : P) / elem_bytes / 8 * 8;
+  t.partial_stride = symmetric ? (len + 7) / 8 * 8 : t.cap;
+  t.gather_stride = symmetric ? 0 : t.cap;
+  return t;
+}
+
 // Bit j set: the partials received at step j are added into what is sent at step t
 // (t == num_steps: into the final result).  Only steps whose received range covers the
 // block in question contribute; the caller checks the range.

@@ -441,6 +441,28 @@ def test_all_reduce_as_reduce_scatter_plus_all_gather_in_one_launch(P, algo, dty
         assert g.size == P
 
 
+@pytest.mark.parametrize("P", [4, 8])
+@pytest.mark.parametrize("algo", [sch.RING, sch.RECURSIVE])
+def test_two_phase_all_reduce_of_private_tensors_shorter_than_the_staging(P, algo):
+    """Launches shorter than the staging area allows, and a last chunk of such a length, while lanes drift apart: the
+    blocks one lane gathers lie beside the partial sums another has not read yet."""
+    staging = 1 << 20
+    comm = pccl.Communicator.emulated_world(P, device=0, heap_bytes=8 << 20, staging_bytes=staging)
+    comm.set_debug(jitter_us=150.0, trace_events=0)
+    cap = pccl._C.two_phase_staging(staging, 4, P, 0, False)[0]
+    for rep in range(3):
+        for blk in (cap // 2 + 3, cap - 9, cap + cap // 2 + 5):
+            ts = [rand(P * blk, torch.float32, 100 * rep + r) for r in range(P)]
+            want = sum(t.double() for t in ts) * 0.5
+            comm.native.all_reduce(comm.world_group.gid, ts, sch.ALGO_IDS[algo], 6, 0.5)
+            comm.check()
+            for r in range(P):
+                torch.testing.assert_close(ts[r].double(), want, rtol=1e-5, atol=1e-5)
+                assert torch.equal(ts[r], ts[0])
+    comm.set_debug(0.0, 0)
+    comm.close()
+
+
 BIG = 9 * (1 << 20) + 24          # elements: > 1 MiB per lane on 4-7 lanes, odd tail, 16-byte aligned start
 
 

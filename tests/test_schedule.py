@@ -117,3 +117,39 @@ def test_header_and_python_agree():
 def test_grid_coords():
     assert sch.grid_coords(5, 2, 2) == (1, 0, 1)
     assert sch.grid_coords(3, 2, 2) == (0, 1, 1)
+
+
+def _lane_bounds(total, gran, lane, lanes):
+    """Range of one lane, as the kernels cut it: equal shares in units of `gran`."""
+    units = -(-total // gran)
+    per = -(-units // lanes)
+    return min(min(per * lane, units) * gran, total), min(min(per * (lane + 1), units) * gran, total)
+
+
+@pytest.mark.parametrize("P", [2, 4, 8])
+@pytest.mark.parametrize("size", [2, 4])
+def test_phases_of_the_two_phase_all_reduce_do_not_overlap_across_lanes(P, size):
+    """Lanes do not wait for one another: what one lane gathers into the staging area must not lie where another lane's
+    partial sums may still be unread, for full launches and for shorter ones."""
+    from pccl.build_kernels import load
+
+    staging, lanes = 1 << 16, 5
+    cap = load().two_phase_staging(staging, size, P, 0, False)[0]
+    assert cap % 8 == 0 and cap > 0
+    for n in sorted({1, 7, 8, 41, cap // P, cap // 2 + 3, cap - cap // P + 5, cap - 1, cap}):
+        got_cap, partial, gather = load().two_phase_staging(staging, size, P, n, False)
+        assert got_cap == cap and partial >= n and gather >= n and (partial * size) % 16 == 0
+        assert max((P - 1) * partial, P * gather) * size <= staging
+        bounds = [_lane_bounds(n, 8, lane, lanes) for lane in range(lanes)]
+        for a in range(lanes):
+            for b in range(lanes):
+                if a == b:
+                    continue
+                for gs in range(P):
+                    for ps in range(P - 1):
+                        lo, hi = max(gs * gather + bounds[a][0], ps * partial + bounds[b][0]), \
+                            min(gs * gather + bounds[a][1], ps * partial + bounds[b][1])
+                        assert lo >= hi, f"lane {a} slot {gs} over lane {b} partial {ps} at length {n}"
+    # symmetric tensors are gathered in place: only the partial sums are staged
+    cap, partial, _ = load().two_phase_staging(staging, size, P, 41, True)
+    assert partial == 48 and (P - 1) * cap * size <= staging
