@@ -274,7 +274,7 @@ __device__ __forceinline__ void epilogue_store32(const GemmArgs& a, const uint32
     for (int v = 0; v < 4; ++v) {
       float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (bias != nullptr) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(bias + col0 + v * 8));     // N % 8 == 0: 16-byte aligned
+        const uint4 q = *reinterpret_cast<const uint4*>(bias + col0 + v * 8);     // N % 8 == 0: 16-byte aligned
         const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -1087,7 +1087,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
       if (bias != nullptr) {
 #pragma unroll
         for (int s = 0; s < 2; ++s)                                    // N % 8 == 0: a pair is inside or outside as a whole
-          if (colw + s * 64 + 2 * lane < a.N) bias_q[s] = __ldg(reinterpret_cast<const uint32_t*>(bias + colw + s * 64) + lane);
+          if (colw + s * 64 + 2 * lane < a.N) bias_q[s] = *(reinterpret_cast<const uint32_t*>(bias + colw + s * 64) + lane);
       }
       // one lane polls the barrier (with a pause between polls: an accumulator takes microseconds),
       // the others wait at the shuffle: 124 fewer threads hammering shared memory beside the MMAs
@@ -1176,7 +1176,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             if (col0 + c * 8 < a.N) {
-              const uint4 uq = __ldg(reinterpret_cast<const uint4*>(urow + c * 8));
+              const uint4 uq = *reinterpret_cast<const uint4*>(urow + c * 8);
               const uint32_t uw[4] = {uq.x, uq.y, uq.z, uq.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -1307,8 +1307,8 @@ __device__ __forceinline__ void tile_reduce_store(const TileArgs& a, uint32_t ti
     if (gr >= a.M || gc >= a.N) continue;                    // N % 8 == 0: a chunk is inside or outside as a whole
     const size_t off = (size_t)gr * a.N + gc;
     uint4 bq = make_uint4(0u, 0u, 0u, 0u), uq = make_uint4(0u, 0u, 0u, 0u);
-    if (a.bias != nullptr) bq = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.bias) + gc));
-    if (a.gelu_grad_of != nullptr) uq = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.gelu_grad_of) + off));
+    if (a.bias != nullptr) bq = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.bias) + gc);
+    if (a.gelu_grad_of != nullptr) uq = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.gelu_grad_of) + off);
     const uint32_t o0 = (uint32_t)(row * (TN * 4) + (((2 * ch) ^ (row & 31)) << 4)), o1 = (uint32_t)(row * (TN * 4) + (((2 * ch + 1) ^ (row & 31)) << 4));
     float4 v0[SPLIT], v1[SPLIT];
 #pragma unroll

@@ -67,7 +67,7 @@ __device__ __forceinline__ float sq8<float>(const uint4& q) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kOptThreads) sq_norm_kernel(const T* __restrict__ x, uint64_t n, float* out) {
+__global__ void __launch_bounds__(kOptThreads) sq_norm_kernel(const T* x, uint64_t n, float* out) {
   __shared__ float red[32];
   pdl_wait();
   pdl_trigger();
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kOptThreads) sq_norm_kernel(const T* __restric
 // so no host synchronisation sits between the norm all-reduce and the update.
 template <typename G>
 __global__ void __launch_bounds__(kOptThreads)
-    adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v, const G* __restrict__ grad,
+    adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v, const G* grad,
                  __nv_bfloat16* __restrict__ param, uint64_t n, AdamWArgs a, const float* total_sq_norm) {
   pdl_wait();
   pdl_trigger();
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kOptThreads)
 __device__ __forceinline__ float exp_diff(float x, float m) { return ex2_hw((x - m) * 1.4426950408889634f); }
 
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* targets,
                                                             float* loss_sum, int64_t rows, int vocab, int64_t row_stride,
                                                             float grad_scale, int64_t ignore_index, int* bad_targets) {
   pdl_wait();

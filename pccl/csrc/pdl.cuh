@@ -6,6 +6,8 @@
 // Rules every kernel launched this way keeps:
 //   * no thread touches global memory before its pdl_wait(), not even to read (its inputs may be on their way, its
 //     outputs may still be read), and no bounded wait on another role starts before it;
+//   * nothing is read through the non-coherent path (__ldg, or a const __restrict__ pointer): that path takes memory to be
+//     constant for the life of the kernel, which here begins while the kernel in front still writes;
 //   * every block calls pdl_wait(), so a kernel never ends before the ones in front of it;
 //   * pdl_trigger(), which lets the next kernel's blocks in, comes after the block owns all it needs (tensor memory among it):
 //     a block that waits must never hold what a running one still has to acquire.

@@ -59,10 +59,10 @@ __device__ __forceinline__ void col_item(const uint4& q, const uint4& uq, __nv_b
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* __restrict__ X, int64_t T, int N,
+__global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* X, int64_t T, int N,
                                                       __nv_bfloat16* __restrict__ out, float* __restrict__ partial,
-                                                      int* __restrict__ counters, const __nv_bfloat16* __restrict__ U,
-                                                      __nv_bfloat16* __restrict__ DU, const __nv_bfloat16* __restrict__ X2) {
+                                                      int* __restrict__ counters, const __nv_bfloat16* U,
+                                                      __nv_bfloat16* __restrict__ DU, const __nv_bfloat16* X2) {
   __shared__ __align__(16) float red[kRowLanes][kColTile];
   __shared__ int s_last;
   pdl_wait();
@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* __
 // Measured with residual and column sums, without the kernel that adds the partials: @@LNB@@.
 template <int D, int RB>
 __global__ void __launch_bounds__(D / 8, 4096 / D)
-    ln_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean,
-                  const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ resid,
+    ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* mean, const float* rstd,
+                  const __nv_bfloat16* gamma, const __nv_bfloat16* resid,
                   __nv_bfloat16* __restrict__ dx, float* __restrict__ pgamma, float* __restrict__ pbeta, float* __restrict__ pdx,
                   int64_t T) {
   pdl_wait();
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(1024) ln_bwd_finalize_kernel(LnBwdFinalizeArgs
   pdl_wait();
   pdl_trigger();
   __shared__ float sa[32][33];
-  const float* __restrict__ part = f.part[blockIdx.y];
+  const float* part = f.part[blockIdx.y];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;                // d is a multiple of 32
   float a = 0.f;
@@ -328,7 +328,7 @@ __device__ __forceinline__ uint4 gelu8(const uint4& q) {
   }
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
-__global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int64_t nvec) {
+__global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* in, uint4* __restrict__ out, int64_t nvec) {
   pdl_wait();
   pdl_trigger();
   const int64_t stride = (int64_t)gridDim.x * 256;
@@ -355,9 +355,9 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__
 // @@LNF@@.
 constexpr int kLnFwdWarps = 4;      // per block: small ones, so that few rows still reach every SM
 template <int D>
-__global__ void __launch_bounds__(32 * kLnFwdWarps, 6) ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* branch,
-                                                        const __nv_bfloat16* __restrict__ gamma,
-                                                        const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(32 * kLnFwdWarps, 6) ln_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* branch,
+                                                        const __nv_bfloat16* gamma, const __nv_bfloat16* beta,
+                                                        __nv_bfloat16* __restrict__ y,
                                                         float* __restrict__ mean, float* __restrict__ rstd, int64_t T, float eps) {
   pdl_wait();
   pdl_trigger();

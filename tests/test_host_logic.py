@@ -474,3 +474,19 @@ def test_sweep_markdown_handles_lane_suffixed_variants():
                      "best": best, "best_without_multimem": best}]}
     text = mod.markdown(doc)
     assert "pull@4 µs" in text and "pull@64 µs" in text and "| 8 | 50.0 |" in text
+
+
+def test_kernels_that_start_early_use_no_non_coherent_loads():
+    """A kernel launched before the one in front of it has ended must not read through the path that takes memory to be
+    constant for the kernel's life: no __ldg, and no pointer the compiler may read that way (const and __restrict__)."""
+    import re
+
+    from pccl.build_kernels import CSRC
+
+    early = [p for p in sorted(CSRC.iterdir()) if p.suffix in (".cu", ".cuh") and re.search(r'#include "pdl.cuh"', p.read_text())]
+    assert {"gemm_sm100.cu", "optim.cu", "train_ops.cu"} <= {p.name for p in early}
+    for p in early:
+        code = re.sub(r"//[^\n]*", "", p.read_text())
+        for pattern in (r"__ldg\s*\(", r"ld\.global\.nc", r"\bconst\s+[\w:]+\s*\*\s*(const\s+)?__restrict__"):
+            found = re.search(pattern, code)
+            assert found is None, f"{p.name}: {found.group(0)}"
