@@ -1,4 +1,6 @@
 """ZeRO-3 engine and training kernels on one GPU."""
+import math
+
 import pytest
 import torch
 
@@ -118,6 +120,25 @@ def test_cross_entropy_rows_per_block_and_ragged_columns(rows, vocab):
         assert float((logits.double() - grad).abs().max()) <= 2.0 ** -8 * 0.25
         assert float((logits.double() - grad).norm() / grad.norm()) < 3e-3
     assert bool((store[:, vocab:] == 7.0).all())
+
+
+@pytest.mark.parametrize("rows,vocab", [(16384, 1024), (16384, 4096), (16384, 16384)])
+def test_cross_entropy_sum_of_many_equal_rows(rows, vocab):
+    """Equal losses round the same way every time they are added to a large sum.  Each block adds up its own rows first, so
+    only the blocks' sums meet the large one: at most half a unit in its last place per block."""
+    import pccl
+
+    logits = torch.zeros(rows, vocab, device=DEV, dtype=torch.bfloat16)
+    targets = torch.arange(rows, device=DEV) % vocab
+    loss = torch.zeros(1, device=DEV)
+    pccl._C.ce_fwd_bwd(logits, targets, loss, 1.0, -100)
+    threads = 512 if vocab >= 16384 else 256 if vocab >= 4096 else 128
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    blocks = min(rows, sms * (1024 // threads))
+    want = rows * math.log(vocab)
+    ulp = 2.0 ** (math.floor(math.log2(want)) - 23)
+    # the blocks' own sums are 64 and more times smaller; a row's logarithm is good to a few units in its last place
+    assert abs(float(loss) - want) <= blocks * ulp / 2 + want * 1e-6
 
 
 def test_cross_entropy_reports_targets_outside_the_vocabulary():
