@@ -133,8 +133,11 @@ void maybe_split_last_wave(GemmArgs& a, int device, cudaStream_t stream) {
   if (a.sk_epoch == 0) a.sk_epoch = ++w.epoch;      // 0 is what fresh flags hold
 }
 
-void fill_common(GemmArgs& a, const at::Tensor& A, const at::Tensor& C, const std::optional<at::Tensor>& bias, int N, int K,
-                 at::Tensor& err) {
+// Returns what has to live until the launch: a copy of a bias that lies where the kernels' loads (pairs of elements in
+// the CTA-pair form, eight in the one-SM form) would be misaligned.
+at::Tensor fill_common(GemmArgs& a, const at::Tensor& A, const at::Tensor& C, const std::optional<at::Tensor>& bias, int N, int K,
+                       at::Tensor& err, bool two_cta) {
+  at::Tensor keep;
   std::memset(&a, 0, sizeof(a));
   a.M = (int)A.size(0);
   a.N = N;
@@ -145,8 +148,11 @@ void fill_common(GemmArgs& a, const at::Tensor& A, const at::Tensor& C, const st
   if (bias.has_value()) {
     TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == at::kBFloat16 && bias->numel() == N && bias->is_contiguous(),
                 "bias must be a contiguous bfloat16 vector of N elements");
-    a.bias = bias->data_ptr();
+    keep = *bias;
+    if (reinterpret_cast<uintptr_t>(keep.data_ptr()) % (two_cta ? 4 : 16) != 0) keep = keep.clone();
+    a.bias = keep.data_ptr();
   }
+  return keep;
 }
 
 // C = A @ W^T (+ bias).  Returns (C, error flag tensor): error stays 0 unless a bounded wait ran out.
@@ -163,7 +169,7 @@ std::tuple<at::Tensor, at::Tensor> gemm(const at::Tensor& A, const at::Tensor& W
   TORCH_CHECK(C.size(0) == A.size(0) && C.size(1) == N, "out has the wrong shape");
   at::Tensor err = error_word(A.get_device());
   GemmArgs a;
-  fill_common(a, A, C, bias, N, K, err);
+  const at::Tensor bias_kept = fill_common(a, A, C, bias, N, K, err, two_cta);
   a.W = W.data_ptr();
   a.two_cta = two_cta ? 1 : 0;
   cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
@@ -193,7 +199,7 @@ at::Tensor gemm_ex(const at::Tensor& A, const at::Tensor& B, bool a_mn, bool b_m
   TORCH_CHECK(C.size(0) == M && C.size(1) == N, "out has the wrong shape");
   at::Tensor err = error_word(A.get_device());
   GemmArgs a;
-  fill_common(a, A, C, bias, N, K, err);
+  const at::Tensor bias_kept = fill_common(a, A, C, bias, N, K, err, true);
   a.M = M;
   a.W = B.data_ptr();
   a.two_cta = 1;
@@ -225,7 +231,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> gemm_gelu(const at::Tensor& A, co
   at::Tensor G = at::empty({A.size(0), N}, A.options());
   at::Tensor err = error_word(A.get_device());
   GemmArgs a;
-  fill_common(a, A, U, bias, N, K, err);
+  const at::Tensor bias_kept = fill_common(a, A, U, bias, N, K, err, two_cta);
   a.W = W.data_ptr();
   a.act_out = G.data_ptr();
   a.two_cta = two_cta ? 1 : 0;
@@ -388,7 +394,7 @@ std::tuple<at::Tensor, at::Tensor> ag_gemm(Comm& c, int gid, const at::Tensor& A
   check_bf16_2d(C, "out");
   at::Tensor err = error_word(dev);
   GemmArgs a;
-  fill_common(a, A, C, bias, N, K, err);
+  const at::Tensor bias_kept = fill_common(a, A, C, bias, N, K, err, two_cta);
   a.W = w_full.data_ptr();
   a.two_cta = two_cta ? 1 : 0;
   a.shard_off = (uint64_t)off;
@@ -429,7 +435,7 @@ std::tuple<at::Tensor, at::Tensor> ag_gemm_local(const at::Tensor& A, std::vecto
   at::Tensor err = error_word(dev);
   at::Tensor flags = at::zeros({N / kGemmBN}, A.options().dtype(at::kInt));
   GemmArgs a;
-  fill_common(a, A, C, bias, N, K, err);
+  const at::Tensor bias_kept = fill_common(a, A, C, bias, N, K, err, two_cta);
   a.W = w_full.data_ptr();
   a.two_cta = two_cta ? 1 : 0;
   a.shard_off = 0;

@@ -1655,6 +1655,7 @@ cudaError_t launch_gemm_sm100(const GemmArgs& a_in, int sm_count, cudaStream_t s
   if ((reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.W) | reinterpret_cast<uintptr_t>(a.C)) & 15u)
     return cudaErrorInvalidValue;
   if (a.act_out != nullptr && (reinterpret_cast<uintptr_t>(a.act_out) & 15u)) return cudaErrorInvalidValue;
+  if (reinterpret_cast<uintptr_t>(a.bias) % (a.two_cta ? 4 : 16) != 0) return cudaErrorInvalidValue;
   const bool fused = a.panel_flags != nullptr;
   if (a.gather_ctas > 0 && !fused) return cudaErrorInvalidValue;
   if (fused && a.gather_ctas == 0 && !a.two_cta) return cudaErrorInvalidValue;   // externally filled panels: CTA-pair form only

@@ -123,6 +123,25 @@ def test_one_tile_per_cta(shape, layout):
     assert C.gemm_pick_tile(8192, 8192, 2048, 148) == (0, 0)
 
 
+@pytest.mark.parametrize("two_cta", [False, True], ids=["one_sm", "cta_pair"])
+@pytest.mark.parametrize("shift", [1, 2, 8])
+@pytest.mark.parametrize("shape", [(256, 768, 256), (1000, 520, 328)])
+def test_bias_that_starts_anywhere(shape, shift, two_cta):
+    """The kernels load the bias in pairs or vectors; a view into a larger buffer may start at any element."""
+    import pccl
+
+    M, N, K = shape
+    a, w = rnd((M, K), 1), rnd((N, K), 2, 0.05)
+    bias = rnd((N + shift,), 3)[shift:]
+    ref = a.float() @ w.float().t() + bias.float()
+    y, err = pccl._C.gemm(a, w, bias, None, two_cta)
+    u, g, err2 = pccl._C.gemm_gelu(a, w, bias, two_cta)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and int(err2.item()) == 0
+    check_close(y, ref, K)
+    assert torch.equal(u, y)
+
+
 def test_linear_wrapper_and_identity():
     from pccl.ops.gemm import linear
 
