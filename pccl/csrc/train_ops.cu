@@ -166,7 +166,11 @@ __global__ void __launch_bounds__(256, 4) col_sum_kernel(const __nv_bfloat16* X,
 // system waits while the block reduces.  One barrier per two rows (the row sums are double-buffered); the
 // arithmetic goes two elements per instruction.  Bound by HBM at many rows, by the chain of row reductions at few.
 // Measured with residual and column sums, without the kernel that adds the partials: @@LNB@@.
-template <int D, int RB>
+// AHEAD false: RB rows at a time, nothing in flight while they are reduced.  At 2048 columns with a residual
+// gradient two blocks share an SM and cover for one another, and three rows of loads at once are worth more than two rows ahead:
+// calls with residual and column sums, ahead / three rows (us): 500 rows 9.1 / 10.0, 1501 13.2 / 13.2, 4096 21.9 / 21.4,
+// 8192 37.4 / 35.0, 32768 116.5 / 103.6.  (One block per SM at 4096 columns, four at 1024: ahead is the better form.)
+template <int D, int RB, bool AHEAD>
 __global__ void __launch_bounds__(D / 8, 4096 / D)
     ln_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* mean, const float* rstd,
                   const __nv_bfloat16* gamma, const __nv_bfloat16* resid,
@@ -207,10 +211,11 @@ __global__ void __launch_bounds__(D / 8, 4096 / D)
   constexpr float inv_d = 1.0f / (float)D;
   const int64_t step = (int64_t)RB * gridDim.x;
   Rows cur, nxt;
-  load(cur, (int64_t)blockIdx.x * RB);
+  if (AHEAD) load(cur, (int64_t)blockIdx.x * RB);
   int buf = 0;
   for (int64_t base = (int64_t)blockIdx.x * RB; base < T; base += step, buf ^= 1) {
-    load(nxt, base + step);
+    if (AHEAD) load(nxt, base + step);
+    else load(cur, base);
     // ---- row sums and the weight/bias gradient sums
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
@@ -269,7 +274,7 @@ __global__ void __launch_bounds__(D / 8, 4096 / D)
         *reinterpret_cast<uint4*>(dx + r * D + t * 8) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
       }
     }
-    cur = nxt;
+    if (AHEAD) cur = nxt;
   }
   auto put = [&](float* row, const F2 (&acc)[4]) {
     float v[8];
@@ -535,11 +540,15 @@ cudaError_t launch_ln_bwd(const void* dy, const void* x, const float* mean, cons
   float* pgamma = scratch;
   float* pbeta = scratch + (int64_t)ln_bwd_blocks(d) * d;
   float* pdx = dx_col_sum != nullptr ? scratch + 2 * (int64_t)ln_bwd_blocks(d) * d : nullptr;
+  auto run = [&](auto* kernel) { return launch_pdl(kernel, blocks, d / 8, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); };
   cudaError_t e = cudaSuccess;
   switch (d / 128) {
-    case 8: e = launch_pdl(ln_bwd_kernel<1024, 2>, blocks, 128, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
-    case 16: e = launch_pdl(ln_bwd_kernel<2048, 2>, blocks, 256, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
-    case 32: e = launch_pdl(ln_bwd_kernel<4096, 2>, blocks, 512, 0, s, DY, X, mean, rstd, G, RS, DX, pgamma, pbeta, pdx, T); break;
+    case 8: e = run(ln_bwd_kernel<1024, 2, true>); break;
+    case 16:
+      // the comment at the kernel has both sides of this line
+      e = resid != nullptr && T >= 4096 ? run(ln_bwd_kernel<2048, 3, false>) : run(ln_bwd_kernel<2048, 2, true>);
+      break;
+    case 32: e = run(ln_bwd_kernel<4096, 2, true>); break;
     default: return cudaErrorInvalidValue;
   }
   if (e != cudaSuccess) return e;
