@@ -96,6 +96,9 @@ constexpr size_t kGemmSkFlagsPerPair = 16;
 // (0: none).  The caller provides scratch for sm_count / 2 pairs when this is non-zero.
 int gemm_sk_tiles(int M, int N, int K, int sm_count);
 
+// Whether that split saves more than it costs.
+bool gemm_split_pays(int M, int N, int K, int sm_count);
+
 // Width and split of the one-tile-per-CTA form for this shape, or 0 and 0 where the CTA-pair kernel is the faster one.
 void gemm_pick_tile(int M, int N, int K, int sm_count, int* tile_n, int* tile_split);
 

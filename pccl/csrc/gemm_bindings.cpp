@@ -58,8 +58,6 @@ bool g_dynamic_tiles = false;  // hand tiles out at run time instead of dealing 
 int g_max_pairs = 0, g_group_m = 0;      // tuning knobs, 0: the kernel's defaults
 int g_wide = -1;                         // units of two row-tiles that share their W half: 1 always, 0 never, -1 where measured faster
 
-constexpr long long kSplitCostNs = 6000;
-
 SkWorkspace& sk_workspace(int device, cudaStream_t stream, int pairs) {
   static std::map<std::pair<int, cudaStream_t>, SkWorkspace> all;
   static std::mutex mu;
@@ -89,9 +87,12 @@ void maybe_split_last_wave(GemmArgs& a, int device, cudaStream_t stream) {
     if (a.tile_n > 0) return;
   }
   if (g_wide != 0 && g_max_pairs == 0 && a.two_cta && a.panel_flags == nullptr && a.M > 256) {
-    // Units of two row-tiles (never split along K).  Measured on the training shapes: 6-28 % faster than
-    // single tiles for contractions of 4096 and more when the units fill their rounds, slower for short
-    // contractions, where the epilogue of a unit (both accumulators) is no longer hidden.
+    // Units of two row-tiles (never split along K), for contractions of 4096 and more when the units fill their
+    // rounds.  Measured with the clocks up, best form of single tiles / units (us): 8192 x 2048 x 8192 190 / 182, 4096 x
+    // 16384 x 4096 393 / 359, 8192 x 4096 x 16384 744 / 727, 6144 x 4096 x 4096 140 / 140; one of the worst on this side of the line
+    // 2816 x 7936 x 4096 130 / 139.  Rounds not filled: 6144 x 2048 x 8192 146 / 165.  Shorter contractions, where the epilogue of a
+    // unit (both accumulators) is not hidden: 4096 x 4096 x 1024 29.2 / 31.5, 8192 x 6144 x 2048 141 / 146, 8192 x 8192 x 2048
+    // 184 / 182.  Under the power cap (launches for seconds) 8192 x 2048 x 8192 226 / 215, 4096 x 16384 x 4096 468 / 424.
     const long long units = (long long)((a.M + 511) / 512) * ((a.N + 255) / 256);
     const long long pairs = sm_count(device) / 2;
     const long long rounds = (units + pairs - 1) / pairs;
@@ -119,12 +120,7 @@ void maybe_split_last_wave(GemmArgs& a, int device, cudaStream_t stream) {
   // fewer tiles than CTA pairs: splitting every tile wins a single cold launch, but back to back under the power
   // cap the unsplit launch is faster (2048 x 2048 x 8192: 65 against 74 us), so it is opt-in
   if ((long long)((a.M + 255) / 256) * ((a.N + 255) / 256) < sms / 2 && !g_split_single_round) return;
-  if (!g_split_single_round) {
-    // The split saves the idle part of the last round and costs the exchange of partial sums.  @@SKCOST@@
-    const long long G = sms / 2, T = (long long)((a.M + 255) / 256) * ((a.N + 255) / 256);
-    const long long rounds = (T + G - 1) / G, nkb = (a.K + 63) / 64;
-    if (281 * nkb * (rounds * G - T) / G < kSplitCostNs) return;
-  }
+  if (!g_split_single_round && !gemm_split_pays(a.M, a.N, a.K, sms)) return;
   SkWorkspace& w = sk_workspace(device, stream, sms / 2);
   a.sk_tiles = n;
   a.sk_scratch = w.scratch.data_ptr<float>();
@@ -473,6 +469,7 @@ void bind_gemm(py::module_& m) {
         "CTA pairs draw their tiles from a counter at run time (robust beside kernels that hold some SMs) instead of a "
         "fixed round-robin share; excludes the split of the last round");
   m.def("gemm_set_tiles", [](bool on) { g_tiles = on; }, "allow the one-tile-per-CTA form (default on)");
+  m.def("gemm_split_pays", &gemm_split_pays, "whether splitting the last round along K is expected to save more than it costs");
   m.def("gemm_pick_tile", [](int M, int N, int K, int sms) {
     int n = 0, s = 0;
     gemm_pick_tile(M, N, K, sms, &n, &s);

@@ -305,6 +305,24 @@ def test_last_round_split_along_k(shape, layout):
         C.gemm_set_wide(-1)
 
 
+@pytest.mark.parametrize("shape", [(2048, 5120, 1024), (5760, 1728, 1536), (2048, 5120, 2048), (3328, 1600, 2056), (2176, 2240, 1544)])
+def test_default_choice_around_the_split_of_the_last_round(shape):
+    """Just below and above the line where the last round is split, by the default rules, launches back to back."""
+    import pccl
+
+    C = pccl._C
+    M, N, K = shape
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert C.gemm_pick_tile(M, N, K, sms) == (0, 0) and C.gemm_sk_tiles(M, N, K, sms) > 0
+    a, w, bias = rnd((M, K), 1), rnd((N, K), 2, 0.05), rnd((N,), 3)
+    ref = a.float() @ w.float().t() + bias.float()
+    ys = [C.gemm_ex(a, w, False, False, bias, None) for _ in range(3)]
+    torch.cuda.synchronize()
+    assert int(C.gemm_error_word(0).item()) == 0
+    check_close(ys[0], ref, K)
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+
+
 @pytest.mark.parametrize("shape", [(512, 768, 256), (960, 512, 328), (8192, 8192, 2048), (1024, 2048, 4096)])
 def test_gemm_with_gelu_backward_epilogue(shape):
     """du = (dy @ W) * gelu'(u): the GELU backward as the epilogue of the data-gradient product (W stored

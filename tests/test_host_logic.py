@@ -476,6 +476,18 @@ def test_sweep_markdown_handles_lane_suffixed_variants():
     assert "pull@4 µs" in text and "pull@64 µs" in text and "| 8 | 50.0 |" in text
 
 
+def test_last_round_is_split_where_its_idle_part_is_worth_the_exchange():
+    """The line on both sides, at full, nearly full and nearly empty last rounds, for large and small products."""
+    import pccl
+
+    pays = pccl._C.gemm_split_pays
+    assert pays(2048, 5120, 2048, 148) and not pays(2048, 5120, 1024, 148)          # 160 tiles: 62 of 74 pairs idle in the last round
+    assert not pays(8192, 6144, 2048, 148) and pays(8192, 6144, 2240, 148)          # 768 tiles, 46 of 74 idle: 35 k-blocks
+    assert not pays(256 * 74, 256, 65536, 148)                                      # full rounds: nothing to save at any length
+    assert not pays(256 * 73, 256, 65536 // 8, 148) and pays(256 * 75, 256, 2048, 148)
+    assert not pays(8, 8, 8, 148) and not pays(8, 8, 8, 1)
+
+
 def test_kernels_that_start_early_use_no_non_coherent_loads():
     """A kernel launched before the one in front of it has ended must not read through the path that takes memory to be
     constant for the kernel's life: no __ldg, and no pointer the compiler may read that way (const and __restrict__)."""
