@@ -526,6 +526,35 @@ def test_copy_engine_paths_carry_bf16(P):
     comm.close()
 
 
+@pytest.mark.parametrize("P", [4, 8])
+@pytest.mark.parametrize("algo", [sch.RING, sch.RECURSIVE])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_middle_steps_sum_through_the_copy_engine(P, algo, dtype):
+    """Ring and halving with more than 192 KiB per lane and block, aligned, not a multiple of the ring's sub-chunks: the
+    partial sums of the middle steps come from staged chunks and go straight into a peer's staging area.  Lanes drift
+    apart between repetitions."""
+    lanes, size = 2, torch.tensor([], dtype=dtype).element_size()
+    n = lanes * (192 * 1024 // size + 4 * 1024) + 1024 + 8
+    comm = pccl.Communicator.emulated_world(P, device=0, heap_bytes=(P + 2) * n * size + (16 << 20), staging_bytes=P * n * size + (1 << 20))
+    comm.set_debug(jitter_us=100.0, trace_events=0)
+    gid = comm.world_group.gid
+    for rep in range(3):
+        ins = [rand(P * n, dtype, 50 * rep + r) for r in range(P)]
+        want = sum(t.double() for t in ins).view(P, n) / P
+        outs = [torch.zeros(n, dtype=torch.float32, device=DEV) for _ in range(P)]
+        comm.native.reduce_scatter(gid, outs, ins, sch.ALGO_IDS[algo], lanes, 1.0 / P, None)
+        both = [t.clone() for t in ins]
+        comm.native.all_reduce(gid, both, sch.ALGO_IDS[algo], lanes, 1.0 / P)
+        comm.check()
+        # fp32: P - 1 roundings of sums of up to P values of size 5; bf16: a rounding of each partial sum on the way
+        tol = dict(rtol=0, atol=P * P * 5 * 2.0 ** -24 / P) if dtype == torch.float32 else dict(rtol=0, atol=P * P * 5 * 2.0 ** -9 / P)
+        for r in range(P):
+            torch.testing.assert_close(outs[r].double(), want[r], **tol)
+            torch.testing.assert_close(both[r].double().view(P, n), want, **tol)
+    comm.set_debug(0.0, 0)
+    comm.close()
+
+
 def test_collectives_of_different_groups_share_the_staging_area_in_order():
     """Two groups of one communicator use the same staging bytes.  An asynchronous all-gather on
     group A (side stream, private output: staged) followed at once by a reduce-scatter on group B
