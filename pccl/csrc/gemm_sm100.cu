@@ -81,6 +81,13 @@ __device__ __forceinline__ bool gemm_wait_relaxed(uint64_t* bar, uint32_t parity
   }
 }
 
+// After a wait that ran out: the last loads issued into a ring of `stages` (numbers [0, issued)) have to land before
+// the CTA may leave its shared memory.  Bounded as a whole, and blind to the abort flag.
+__device__ __noinline__ void drain_loads(uint64_t* full, uint32_t issued, uint32_t stages) {
+  for (uint32_t n = issued > stages ? issued - stages : 0; n < issued; ++n)
+    mbar_wait(full + n % stages, (n / stages) & 1u, kWaitNs / stages);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -414,7 +421,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         tma_load_2d(sa + kABytes, wmap, kb * BK, wy, full + s);
       }
     }
-    if (!ok) *abort_flag = 1;
+    // see every load land: all stages given back, or (a wait ran out) the loads themselves
+    for (uint32_t n = it > (uint32_t)kStages ? it - kStages : 0; ok && n < it; ++n)
+      ok = gemm_wait(empty + n % kStages, (n / kStages) & 1u, abort_flag);
+    if (!ok) {
+      *abort_flag = 1;
+      drain_loads(full, it, kStages);
+    }
   } else if (warp == 1 && lane == 0) {
     // ------------------------------------------------------------ MMA issuer
     uint32_t it = 0, tile_count = 0;
@@ -964,6 +977,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemm2Threads, 1)
     if (!ok) {
       atomicCAS(a.error, 0, kErrProducer);
       *abort_flag = 1;
+      if (leader) drain_loads(full, it, NST);       // both CTAs' loads count on the leader's barriers, and both meet below
     }
   } else if (warp == 1 && lane == 0 && leader) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
@@ -1401,6 +1415,7 @@ __global__ void __launch_bounds__(kTileThreads, TileCfg<TN>::kPerSm)
   pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
+  uint32_t issued = (uint32_t)(n < Cfg::kStages ? n : Cfg::kStages);      // thread 0's loads so far
   if (warp == 0 && lane == 0) {
     int s = 0;
     uint32_t ph = 0;
@@ -1411,6 +1426,7 @@ __global__ void __launch_bounds__(kTileThreads, TileCfg<TN>::kPerSm)
         break;
       }
       load(i, s);
+      ++issued;
       if (++s == Cfg::kStages) {
         s = 0;
         ph ^= 1u;
@@ -1464,6 +1480,7 @@ __global__ void __launch_bounds__(kTileThreads, TileCfg<TN>::kPerSm)
   } else if (lane == 0) {
     atomicCAS(a.error, 0, kErrEpilogue);
     *abort_flag = 1;
+    if (warp == 0) drain_loads(full, issued, Cfg::kStages);
   }
   tc_fence_before();
   __syncwarp();
