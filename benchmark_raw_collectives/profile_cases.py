@@ -5,7 +5,7 @@
     python benchmark_raw_collectives/profile_cases.py reduce_scatter
     python benchmark_raw_collectives/profile_cases.py adamw
     python benchmark_raw_collectives/profile_cases.py cross_entropy
-    python benchmark_raw_collectives/profile_cases.py gemm_nn | gemm_tn | gemm_split | cublas_gemm
+    python benchmark_raw_collectives/profile_cases.py gemm_nn | gemm_tn | gemm_split | gemm_tile | cublas_gemm
     python benchmark_raw_collectives/profile_cases.py all_gather_ring | all_gather_recursive
     python benchmark_raw_collectives/profile_cases.py reduce_scatter_ring | reduce_scatter_recursive
     python benchmark_raw_collectives/profile_cases.py all_reduce | all_reduce_ring | broadcast
@@ -150,6 +150,17 @@ def gemm_tn():
     torch.cuda.synchronize()
 
 
+def gemm_tile():
+    """One 128-row tile per CTA, the contraction split over clusters: data gradient of an output projection, 2048 tokens."""
+    M, N, K = 2048, 1024, 50304
+    dy = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    W = (torch.randn(K, N, device=DEV) * 0.02).to(torch.bfloat16)
+    out = torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    for _ in range(3):
+        pccl._C.gemm_ex(dy, W, False, True, None, out)
+    torch.cuda.synchronize()
+
+
 def gemm_split():
     """64 tiles on 74 CTA pairs: every tile is split along K and finished from fp32 partial sums."""
     M, N, K = 2048, 2048, 8192
@@ -246,6 +257,7 @@ def col_sum():
 CASES = {
     "gemm": gemm, "cublas_gemm": cublas_gemm, "gemm_proj": gemm_proj, "cublas_gemm_proj": lambda: gemm_proj(True),
     "gemm_wide": gemm_wide, "gemm_nn": gemm_nn, "gemm_tn": gemm_tn, "gemm_split": gemm_split,
+    "gemm_tile": gemm_tile,
     "all_gather": all_gather, "all_gather_ring": lambda: _ag(sch.RING), "all_gather_recursive": lambda: _ag(sch.RECURSIVE),
     "reduce_scatter": reduce_scatter, "reduce_scatter_ring": lambda: _rs(sch.RING),
     "reduce_scatter_recursive": lambda: _rs(sch.RECURSIVE),
