@@ -282,6 +282,26 @@ def test_col_sum_matches_fp32_reference(shape):
         torch.testing.assert_close(out.float(), ref, rtol=1e-2, atol=1e-2 * float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("shape", [(16384, 264), (16385, 264), (70001, 8), (40000, 1032)])
+def test_column_sums_of_many_rows(shape):
+    """Around the line above which the slices of the rows are no longer few, plain and with the GELU backward."""
+    import pccl
+
+    T, N = shape
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+    x, u = (torch.randn(T, N, device=DEV, generator=g).bfloat16() for _ in range(2))
+    out, gb = (torch.full((N,), 7.0, device=DEV).bfloat16() for _ in range(2))
+    ur = u.double().requires_grad_()
+    torch.nn.functional.gelu(ur, approximate="tanh").backward(x.double())
+    for _ in range(2):                                     # the counters are ready for the next call
+        pccl._C.col_sum(x, out)
+        du = pccl._C.gelu_bwd_col_sum(x, u, gb)
+        # fp32 sums of T values of size 1 (error about sqrt(T) * 2^-24 of their running size), one rounding to bf16
+        for got, want in ((out, x.double().sum(0)), (gb, du.double().sum(0))):
+            assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + T * 2.0 ** -24).all())
+        assert float((du.double() - ur.grad).norm() / ur.grad.norm()) < 3e-3
+
+
 @pytest.mark.parametrize("shape", [(8192, 2048), (333, 1024), (4096, 4096), (1, 2048), (1237, 2048)])
 def test_layer_norm_backward_matches_fp32_reference(shape):
     import pccl
