@@ -50,6 +50,9 @@ SOURCES = [
     "comm.cpp",
     "segments.cpp",
     "collectives.cu",
+    "all_reduce_two_phase_bf16.cu",
+    "all_reduce_two_phase_f16.cu",
+    "all_reduce_two_phase_f32.cu",
     "reduce_scatter_bf16.cu",
     "reduce_scatter_f16.cu",
     "reduce_scatter_f32.cu",

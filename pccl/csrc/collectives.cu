@@ -1,4 +1,4 @@
-// The all-gather, one-shot all-reduce, broadcast and barrier kernels, and the launchers of all collectives.
+// The all-gather, one-shot all-reduce, broadcast and barrier kernels, and the choice of a reduce-scatter kernel.
 #include "collectives.cuh"
 
 namespace pccl {
@@ -171,12 +171,27 @@ static bool rs_ragged(const ReduceScatterArgs& a) {
   for (int i = 0; i < a.g.nlocal; ++i) m |= (uint64_t)reinterpret_cast<uintptr_t>(a.in[i]) | (uint64_t)reinterpret_cast<uintptr_t>(a.out[i]);
   return (m & 15u) != 0;
 }
+
+// The middle steps of the ring and halving schedules add one or two staged blocks to one of their own.  With little data
+// the sums come from L2 and the thread loops are faster; once the inputs of this device's ranks exceed what L2 holds
+// (126 MB) the copy engine keeps more loads in flight, for 16-bit types only.  Halving over eight ranks, with two staged sources in
+// its last step, gains from half of that on.  It is a kernel of its own because either path costs the other 4-7 % beside it in
+// one kernel (registers).  Measured on one device, thread loops / copy engine (us): 4 ranks, ring, 16 lanes of
+// 200 KB / 700 KB / 4 MB 80 / 95, 224 / 213, 1181 / 992; 8 ranks, halving, 8 lanes of 200 KB / 700 KB 147 / 146, 437 / 376; 8 ranks, halving,
+// 18 lanes of 700 KB 525 / 436; fp32, 8 ranks, ring, 8 lanes of 700 KB 314 / 355.
+RsForm rs_form(const ReduceScatterArgs& a) {
+  if (rs_ragged(a)) return kRsRagged;
+  if (a.in_dtype == kF32 || a.wire_dtype != a.in_dtype || (a.algo != kRing && a.algo != kRecursive)) return kRsAligned;
+  const uint64_t bytes = (uint64_t)a.g.nlocal * a.g.size * a.nsub * a.sub_elems * dtype_size(a.in_dtype);
+  const uint64_t line = a.algo == kRecursive && a.g.size >= 8 ? 80ull << 20 : 160ull << 20;
+  return bytes > line ? kRsStreamed : kRsAligned;
+}
 cudaError_t launch_reduce_scatter(const ReduceScatterArgs& a, int nlanes, cudaStream_t stream) {
   if (a.stage_elems < a.sub_elems) return cudaErrorInvalidValue;
-  const bool ragged = rs_ragged(a);
-  if (a.in_dtype == kBF16) return launch_reduce_scatter_bf16(a, ragged, nlanes, stream);
-  if (a.in_dtype == kF16) return launch_reduce_scatter_f16(a, ragged, nlanes, stream);
-  if (a.in_dtype == kF32) return launch_reduce_scatter_f32(a, ragged, nlanes, stream);
+  const RsForm form = rs_form(a);
+  if (a.in_dtype == kBF16) return launch_reduce_scatter_bf16(a, form, nlanes, stream);
+  if (a.in_dtype == kF16) return launch_reduce_scatter_f16(a, form, nlanes, stream);
+  if (a.in_dtype == kF32) return launch_reduce_scatter_f32(a, form, nlanes, stream);
   return cudaErrorInvalidValue;
 }
 
@@ -188,10 +203,10 @@ cudaError_t launch_all_reduce(const AllReduceArgs& a, int nlanes, cudaStream_t s
 }
 cudaError_t launch_all_reduce_rsag(const AllReduceRsAgArgs& a, int nlanes, cudaStream_t stream) {
   if (a.rs.stage_elems < a.rs.sub_elems) return cudaErrorInvalidValue;
-  const bool ragged = rs_ragged(a.rs);
-  if (a.rs.in_dtype == kBF16) return launch_all_reduce_rsag_bf16(a, ragged, nlanes, stream);
-  if (a.rs.in_dtype == kF16) return launch_all_reduce_rsag_f16(a, ragged, nlanes, stream);
-  if (a.rs.in_dtype == kF32) return launch_all_reduce_rsag_f32(a, ragged, nlanes, stream);
+  const RsForm form = rs_form(a.rs);
+  if (a.rs.in_dtype == kBF16) return launch_all_reduce_rsag_bf16(a, form, nlanes, stream);
+  if (a.rs.in_dtype == kF16) return launch_all_reduce_rsag_f16(a, form, nlanes, stream);
+  if (a.rs.in_dtype == kF32) return launch_all_reduce_rsag_f32(a, form, nlanes, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -17,8 +17,9 @@
 // The reference's fp32 vectorAdd launch per step (pccl/src/common.cu:5-19) does not exist
 // here: partial sums are formed in fp32 registers while the data is on its way.
 //
-// A header because reduce-scatter and the two-phase all-reduce are compiled once per input type in sources of their own
-// (reduce_scatter_{bf16,f16,f32}.cu), side by side: all in one source they take twice as long as everything else.
+// A header because reduce-scatter (reduce_scatter_{bf16,f16,f32}.cu) and the two-phase all-reduce
+// (all_reduce_two_phase_{bf16,f16,f32}.cu) are compiled in sources of their own, side by side: all in one source they take twice as long
+// as everything else.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -257,8 +258,9 @@ __device__ __forceinline__ bool lane_reduce(BulkPipe& pipe, char* out, const cha
   return true;
 }
 
-template <int TIN, int TW, int TOUT, bool RAGGED>
+template <int TIN, int TW, int TOUT, RsForm FORM>
 __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, BulkPipe& pipe, uint32_t coll) {
+  constexpr bool RAGGED = FORM == kRsRagged;
   const GroupDev& g = a.g;
   const int P = g.size;
   const LaneCtx c{(int)blockIdx.y, g.first_local + (int)blockIdx.y, (int)blockIdx.x, coll};
@@ -392,8 +394,10 @@ __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, 
           char* d = stage_ptr(s.dst, rs_stage_offset(algo, P, t) + (b - s.send_first), j);
           if (nw == 0 && TW == TIN) {
             if (!lane_copy1<false, RAGGED>(pipe, d, in_ptr(in, b, j), cnt * SI)) return;
-          } else if (!lane_reduce<TIN, TW, TW, true, RAGGED>(pipe, d, in_ptr(in, b, j), w, nw, cnt, 1.0f)) {
-            return;
+          } else if constexpr (FORM == kRsStreamed) {
+            if (!lane_reduce<TIN, TW, TW, true, RAGGED>(pipe, d, in_ptr(in, b, j), w, nw, cnt, 1.0f)) return;
+          } else {
+            cta_reduce<TIN, TW, TW, true, RAGGED>(&d, 1, in_ptr(in, b, j), w, nw, cnt, 1.0f);
           }
         } else {
           if (!lane_reduce<TIN, TW, TOUT, true, RAGGED>(pipe, out_ptr(j), in_ptr(in, b, j), w, nw, cnt, a.scale)) return;
@@ -403,32 +407,12 @@ __device__ __forceinline__ void reduce_scatter_body(const ReduceScatterArgs& a, 
   }
 }
 
-template <int TIN, int TW, int TOUT, bool RAGGED>
+template <int TIN, int TW, int TOUT, RsForm FORM>
 __global__ void __launch_bounds__(kCollThreads, 1) reduce_scatter_kernel(const __grid_constant__ ReduceScatterArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   BulkPipe pipe;
   bulk_pipe_init(pipe, smem, a.g.timeout_ns);
-  reduce_scatter_body<TIN, TW, TOUT, RAGGED>(a, pipe, kCollReduceScatter);
-}
-
-// ============================================================================ all-reduce = reduce-scatter + all-gather
-// The composition the reference's all-reduce uses (pccl/src/yacl.cpp:146-177: reduce-scatter into
-// a temporary, all-gather back; recursive halving + recursive doubling, or ring + ring), as ONE
-// launch: phase one leaves this rank's block of the sum in its slot of the tensor, phase two is
-// the all-gather of those slots with the same schedule family.  The two phases are two calls as
-// far as the flags go (consecutive call numbers), so a step flag of phase one can never be taken
-// for one of phase two; a peer's block is pushed into this rank's tensor only after this rank has
-// signalled its entry into phase two, that is after it has read all of its own input.
-// Lanes keep the same element range in both phases (lane ranges are multiples of 8 elements).
-template <int DT, bool RAGGED>
-__global__ void __launch_bounds__(kCollThreads, 1) all_reduce_rsag_kernel(const __grid_constant__ AllReduceRsAgArgs a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  BulkPipe pipe;
-  bulk_pipe_init(pipe, smem, a.rs.g.timeout_ns);
-  reduce_scatter_body<DT, DT, DT, RAGGED>(a.rs, pipe, kCollAllReduce);
-  cta_bulk_flush(pipe);          // the block written by phase one is what phase two sends
-  __syncthreads();
-  all_gather_body(a.ag, pipe, 8 * Elem<DT>::size, kCollAllReduce);
+  reduce_scatter_body<TIN, TW, TOUT, FORM>(a, pipe, kCollReduceScatter);
 }
 
 template <typename Args>
@@ -455,6 +439,26 @@ cudaError_t launch(void (*kernel)(const Args), const Args& args, int nlanes, int
   return cudaGetLastError();
 }
 
+// ============================================================================ all-reduce = reduce-scatter + all-gather
+// The composition the reference's all-reduce uses (pccl/src/yacl.cpp:146-177: reduce-scatter into
+// a temporary, all-gather back; recursive halving + recursive doubling, or ring + ring), as ONE
+// launch: phase one leaves this rank's block of the sum in its slot of the tensor, phase two is
+// the all-gather of those slots with the same schedule family.  The two phases are two calls as
+// far as the flags go (consecutive call numbers), so a step flag of phase one can never be taken
+// for one of phase two; a peer's block is pushed into this rank's tensor only after this rank has
+// signalled its entry into phase two, that is after it has read all of its own input.
+// Lanes keep the same element range in both phases (lane ranges are multiples of 8 elements).
+template <int DT, RsForm FORM>
+__global__ void __launch_bounds__(kCollThreads, 1) all_reduce_rsag_kernel(const __grid_constant__ AllReduceRsAgArgs a) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  BulkPipe pipe;
+  bulk_pipe_init(pipe, smem, a.rs.g.timeout_ns);
+  reduce_scatter_body<DT, DT, DT, FORM>(a.rs, pipe, kCollAllReduce);
+  cta_bulk_flush(pipe);          // the block written by phase one is what phase two sends
+  __syncthreads();
+  all_gather_body(a.ag, pipe, 8 * Elem<DT>::size, kCollAllReduce);
+}
+
 // The two-phase kernel carries two argument blocks; its group geometry is that of the first.
 cudaError_t launch_rsag(void (*kernel)(const AllReduceRsAgArgs), const AllReduceRsAgArgs& args, int nlanes, cudaStream_t stream) {
   dim3 grid(nlanes, args.rs.g.nlocal), block(kCollThreads);
@@ -476,31 +480,37 @@ cudaError_t launch_rsag(void (*kernel)(const AllReduceRsAgArgs), const AllReduce
 }
 
 // ============================================================================ launches, by the input's type
-// DT: the type of the input, which each source below instantiates for itself (launch.h names the results).
+// DT: the type of the input, which each source instantiates for itself (launch.h names the results).
 template <int DT, int TW, int TOUT>
-cudaError_t launch_rs(const ReduceScatterArgs& a, bool ragged, int nlanes, cudaStream_t stream) {
-  return ragged ? launch(reduce_scatter_kernel<DT, TW, TOUT, true>, a, nlanes, kCollThreads, kBulkSmemBytes, stream)
-                : launch(reduce_scatter_kernel<DT, TW, TOUT, false>, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
+cudaError_t launch_rs(const ReduceScatterArgs& a, RsForm form, int nlanes, cudaStream_t stream) {
+  if (form == kRsRagged) return launch(reduce_scatter_kernel<DT, TW, TOUT, kRsRagged>, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
+  if constexpr (DT == TW && DT != kF32) {      // rs_form never asks for it elsewhere
+    if (form == kRsStreamed) return launch(reduce_scatter_kernel<DT, TW, TOUT, kRsStreamed>, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
+  }
+  return launch(reduce_scatter_kernel<DT, TW, TOUT, kRsAligned>, a, nlanes, kCollThreads, kBulkSmemBytes, stream);
 }
 template <int DT>
-cudaError_t launch_reduce_scatter_of(const ReduceScatterArgs& a, bool ragged, int nlanes, cudaStream_t stream) {
+cudaError_t launch_reduce_scatter_of(const ReduceScatterArgs& a, RsForm form, int nlanes, cudaStream_t stream) {
   const int w = a.wire_dtype, o = a.out_dtype;
   if constexpr (DT == kF32) {
-    if (w == kF32 && o == kF32) return launch_rs<kF32, kF32, kF32>(a, ragged, nlanes, stream);
-    if (w == kF32 && o == kBF16) return launch_rs<kF32, kF32, kBF16>(a, ragged, nlanes, stream);
+    if (w == kF32 && o == kF32) return launch_rs<kF32, kF32, kF32>(a, form, nlanes, stream);
+    if (w == kF32 && o == kBF16) return launch_rs<kF32, kF32, kBF16>(a, form, nlanes, stream);
   } else {
-    if (w == DT && o == DT) return launch_rs<DT, DT, DT>(a, ragged, nlanes, stream);
-    if (w == DT && o == kF32) return launch_rs<DT, DT, kF32>(a, ragged, nlanes, stream);
-    if (w == kF32 && o == DT) return launch_rs<DT, kF32, DT>(a, ragged, nlanes, stream);
-    if (w == kF32 && o == kF32) return launch_rs<DT, kF32, kF32>(a, ragged, nlanes, stream);
+    if (w == DT && o == DT) return launch_rs<DT, DT, DT>(a, form, nlanes, stream);
+    if (w == DT && o == kF32) return launch_rs<DT, DT, kF32>(a, form, nlanes, stream);
+    if (w == kF32 && o == DT) return launch_rs<DT, kF32, DT>(a, form, nlanes, stream);
+    if (w == kF32 && o == kF32) return launch_rs<DT, kF32, kF32>(a, form, nlanes, stream);
   }
   return cudaErrorInvalidValue;
 }
 
 template <int DT>
-cudaError_t launch_all_reduce_rsag_of(const AllReduceRsAgArgs& a, bool ragged, int nlanes, cudaStream_t stream) {
-  return ragged ? launch_rsag(all_reduce_rsag_kernel<DT, true>, a, nlanes, stream)
-                : launch_rsag(all_reduce_rsag_kernel<DT, false>, a, nlanes, stream);
+cudaError_t launch_all_reduce_rsag_of(const AllReduceRsAgArgs& a, RsForm form, int nlanes, cudaStream_t stream) {
+  if (form == kRsRagged) return launch_rsag(all_reduce_rsag_kernel<DT, kRsRagged>, a, nlanes, stream);
+  if constexpr (DT != kF32) {
+    if (form == kRsStreamed) return launch_rsag(all_reduce_rsag_kernel<DT, kRsStreamed>, a, nlanes, stream);
+  }
+  return launch_rsag(all_reduce_rsag_kernel<DT, kRsAligned>, a, nlanes, stream);
 }
 
 }  // namespace
