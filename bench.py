@@ -68,7 +68,7 @@ def parse_args():
     ap.add_argument("--nvls", type=int, default=int(os.environ.get("PCCL_ENABLE_NVLS", "1")),
                     help="bind an NVLS multicast mapping where the machine offers one (the multimem variants win the small sizes)")
     ap.add_argument("--gemm", default=os.environ.get("PCCL_GEMM", "auto"), choices=["auto", "pccl", "cublas"],
-                    help="library arm: auto = plain dense products on cuBLAS (measured 7 %% faster per step than the "
+                    help="library arm: auto = plain dense products on cuBLAS (measured 5 %% faster per step than the "
                          "repository's tcgen05 GEMM) and the fused products (all-gather+GEMM, GEMM+GELU) on the "
                          "repository's kernel, with one more arm that routes every product through it; "
                          "pccl = every product on the repository's GEMM; cublas = none")

@@ -52,7 +52,7 @@ struct SkWorkspace {
   uint32_t next_base = 0;
 };
 bool g_split_last_wave = true;
-bool g_split_single_round = false;        // also split shapes with fewer tiles than CTA pairs (slower back to back: measured)
+bool g_split_single_round = false;        // also split shapes with fewer tiles than CTA pairs
 bool g_tiles = true;           // one tile per CTA where it is the faster form
 bool g_dynamic_tiles = false;  // hand tiles out at run time instead of dealing them out in advance
 int g_max_pairs = 0, g_group_m = 0;      // tuning knobs, 0: the kernel's defaults
@@ -117,8 +117,9 @@ void maybe_split_last_wave(GemmArgs& a, int device, cudaStream_t stream) {
   const int sms = sm_count(device);
   const int n = gemm_sk_tiles(a.M, a.N, a.K, sms);
   if (n <= 0) return;
-  // fewer tiles than CTA pairs: splitting every tile wins a single cold launch, but back to back under the power
-  // cap the unsplit launch is faster (2048 x 2048 x 8192: 65 against 74 us), so it is opt-in
+  // fewer tiles than CTA pairs (and not the one-tile-per-CTA form): splitting every tile through memory is opt-in.  Unsplit / split
+  // (us): 2048 x 2048 x 8192 50 / 58, 4096 x 1024 x 4096 27.9 / 34.5, 2048 x 2048 x 2048 17.3 / 24.1; 3072 x 1024 x 8192 49.0 / 45.8 with the
+  // clocks up, 53.0 / 53.6 under the power cap
   if ((long long)((a.M + 255) / 256) * ((a.N + 255) / 256) < sms / 2 && !g_split_single_round) return;
   if (!g_split_single_round && !gemm_split_pays(a.M, a.N, a.K, sms)) return;
   SkWorkspace& w = sk_workspace(device, stream, sms / 2);
